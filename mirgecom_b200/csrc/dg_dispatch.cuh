@@ -70,9 +70,13 @@ inline int upload_refops_local(int dim, int order, const double* packed64, const
   const int foff = fnodes_offset(dim, order);
   const int fn = fnodes_size(dim, order);
   if (off < 0) return MGC_E_UNSUPPORTED;
-  if (cudaMemcpyToSymbol(c_ref64, packed64, n * sizeof(double), off * sizeof(double)) != cudaSuccess)
+  if (cudaMemcpyToSymbol(g_refops, packed64, n * sizeof(double), off * sizeof(double)) != cudaSuccess)
     return MGC_E_CUDA;
-  if (cudaMemcpyToSymbol(c_ref32, packed32, n * sizeof(float), off * sizeof(float)) != cudaSuccess)
+  const int ng = refgeo_size(dim), goff = refgeo_offset(dim, order);
+  if (cudaMemcpyToSymbol(c_refgeo64, packed64 + n, ng * sizeof(double), goff * sizeof(double)) !=
+          cudaSuccess ||
+      cudaMemcpyToSymbol(c_refgeo32, packed32 + n, ng * sizeof(float), goff * sizeof(float)) !=
+          cudaSuccess)
     return MGC_E_CUDA;
   if (cudaMemcpyToSymbol(c_fnodes, fnodes, fn * sizeof(int), foff * sizeof(int)) != cudaSuccess)
     return MGC_E_CUDA;

@@ -492,12 +492,12 @@ __global__ void __launch_bounds__(256, (Cfg<R, DIM, ORDER, NS, MIX>::MINB_GRAD))
   // reference operators (zero padded; hi/lo tf32 split on the mixed path)
   for (int i = threadIdx.x; i < AWN; i += blockDim.x) {
     const int r = i / (MP * KU), row = (i / KU) % MP, k = i % KU;
-    put_a<R>(aw, AWN, i, (row < NP && k < NP) ? c_ref64[S::OFF_W + (r * NP + row) * NP + k] : 0.0);
+    put_a<R>(aw, AWN, i, (row < NP && k < NP) ? refop(S::OFF_W + (r * NP + row) * NP + k) : 0.0);
   }
   for (int i = threadIdx.x; i < ALN; i += blockDim.x) {
     const int f = i / (MP * KL), row = (i / KL) % MP, m = i % KL;
     put_a<R>(al, ALN, i,
-             (row < NP && m < NFP) ? c_ref64[S::OFF_LIFT + row * NFN + f * NFP + m] : 0.0);
+             (row < NP && m < NFP) ? refop(S::OFF_LIFT + row * NFN + f * NFP + m) : 0.0);
   }
   // padding rows/columns of the B operands stay zero for the whole kernel
   for (int i = threadIdx.x; i < NCOL * (KU + KS); i += blockDim.x) bu[i] = R(0);
@@ -832,9 +832,9 @@ __global__ void __launch_bounds__(256, (Cfg<R, DIM, ORDER, NS, MIX>::MINB))
     if (row < NP && k < KR) {
       if (k < DIM * NP) {
         const int r = k / NP, kk = k % NP;
-        v = -c_ref64[S::OFF_W + (r * NP + row) * NP + kk];
+        v = -refop(S::OFF_W + (r * NP + row) * NP + kk);
       } else {
-        v = c_ref64[S::OFF_LIFT + row * NFN + (k - DIM * NP)];
+        v = refop(S::OFF_LIFT + row * NFN + (k - DIM * NP));
       }
     }
     put_a<R>(am, MP * KB, i, v);
@@ -1388,9 +1388,9 @@ __global__ void __launch_bounds__(256, (Cfg<R, DIM, ORDER, NS, MIX>::MINB_SURF))
     if (row < NP && k < KR) {
       if (k < DIM * NP) {
         const int r = k / NP, kk = k % NP;
-        v = -c_ref64[S::OFF_W + (r * NP + row) * NP + kk];
+        v = -refop(S::OFF_W + (r * NP + row) * NP + kk);
       } else {
-        v = c_ref64[S::OFF_LIFT + row * NFN + (k - DIM * NP)];
+        v = refop(S::OFF_LIFT + row * NFN + (k - DIM * NP));
       }
     }
     put_a<R>(am, MP * KB, i, v);

@@ -1,14 +1,19 @@
-// Reference-element operators of the nodal DG discretization, held in
-// constant memory so that the fully unrolled contractions read them as
-// instruction operands (one broadcast per warp, no shared-memory traffic).
+// Reference-element operators of the nodal DG discretization.
 //
-// For every supported (dim, order) the packed block holds, in order:
+// For every supported (dim, order) the host packs, in order:
 //   W     [dim][Np][Np]   W_r = M^-1 D_r^T M          (weak derivative)
 //   LIFT  [Np][Nf*Nfp]    M^-1 E                      (face lift)
 //   NREF  [Nf][dim]       unit outward reference normals
 //   FSR   [Nf]            reference face measure / face-parametrisation measure
-// The host computes them once (refelem.py) and uploads them through
-// mgc_upload_reference_operators().
+// (refelem.py; mgc_upload_reference_operators()).
+//
+// The matrices W and LIFT live in a global-memory table: every kernel reads
+// them once per CTA, one entry per thread, to build its tensor-core operands
+// in shared memory.  (From constant memory those per-lane addresses replay one
+// by one; one call of the reacting p3 right-hand side on 1260 tetrahedra,
+// float32: 90.6 us from constant memory, 86.1 us from the table, the 24^3 p3
+// Taylor-Green one in float64 830 and 824 us.)  NREF and FSR, a few values
+// each thread reads for its face, stay in constant memory.
 #pragma once
 #include <cstdint>
 
@@ -21,11 +26,13 @@ __host__ __device__ constexpr int simplex_npts(int dim, int order) {
                   : (order + 1) * (order + 2) * (order + 3) / 6;
 }
 
+// matrices of one (dim, order): W, LIFT
 __host__ __device__ constexpr int refops_size(int dim, int order) {
   return dim * simplex_npts(dim, order) * simplex_npts(dim, order) +
-         simplex_npts(dim, order) * (dim + 1) * simplex_npts(dim - 1, order) +
-         (dim + 1) * dim + (dim + 1);
+         simplex_npts(dim, order) * (dim + 1) * simplex_npts(dim - 1, order);
 }
+// NREF, FSR
+__host__ __device__ constexpr int refgeo_size(int dim) { return (dim + 1) * dim + (dim + 1); }
 
 // supported simplex discretizations, in packing order
 __host__ __device__ constexpr int refops_slot(int dim, int order) {
@@ -49,11 +56,20 @@ __host__ __device__ constexpr int refops_offset(int dim, int order) {
 
 constexpr int kRefOpsTotal = refops_offset(3, 3) + refops_size(3, 3);
 
+constexpr int kRefGeoStride = refgeo_size(3);
+constexpr int kRefGeoTotal = (refops_slot(3, 3) + 1) * kRefGeoStride;
+__host__ __device__ constexpr int refgeo_offset(int dim, int order) {
+  return refops_slot(dim, order) * kRefGeoStride;
+}
+
 // Every translation unit that launches kernels holds its own copy (internal
 // linkage, no relocatable device code); mgc_upload_reference_operators()
 // fills the copy of each unit.
-static __constant__ double c_ref64[kRefOpsTotal];
-static __constant__ float c_ref32[kRefOpsTotal];
+static __device__ double g_refops[kRefOpsTotal];
+static __constant__ double c_refgeo64[kRefGeoTotal];
+static __constant__ float c_refgeo32[kRefGeoTotal];
+
+__device__ __forceinline__ double refop(int i) { return __ldg(g_refops + i); }
 
 __host__ __device__ constexpr int fnodes_size(int dim, int order) {
   return (dim + 1) * simplex_npts(dim - 1, order);
@@ -90,17 +106,17 @@ struct Simplex {
   static constexpr int OFF = refops_offset(DIM, ORDER);
   static constexpr int OFF_W = OFF;
   static constexpr int OFF_LIFT = OFF_W + DIM * NP * NP;
-  static constexpr int OFF_NREF = OFF_LIFT + NP * NF * NFP;
+  static constexpr int OFF_NREF = refgeo_offset(DIM, ORDER);
   static constexpr int OFF_FSR = OFF_NREF + NF * DIM;
   static_assert(OFF >= 0, "unsupported simplex discretization");
 };
 
 template <class R> struct RefBank;
 template <> struct RefBank<double> {
-  static __device__ __forceinline__ double get(int i) { return c_ref64[i]; }
+  static __device__ __forceinline__ double get(int i) { return c_refgeo64[i]; }
 };
 template <> struct RefBank<float> {
-  static __device__ __forceinline__ float get(int i) { return c_ref32[i]; }
+  static __device__ __forceinline__ float get(int i) { return c_refgeo32[i]; }
 };
 
 }  // namespace mgc

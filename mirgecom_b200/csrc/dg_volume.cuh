@@ -285,6 +285,20 @@ __device__ __forceinline__ void store_rec(R* dst, const R (&rec)[TW]) {
   }
 }
 
+// Face slots f * NFP + m of each volume node (-1: none), [NP][NF], in face
+// order: one node per thread, every thread of a warp reading the same face
+// node at a time.
+template <int DIM, int ORDER>
+__device__ __forceinline__ void fill_slots(int16_t* slot_s) {
+  using S = Simplex<DIM, ORDER>;
+  for (int k = threadIdx.x; k < S::NP; k += blockDim.x) {
+    int n = 0;
+    for (int fm = 0; fm < S::NF * S::NFP; ++fm)
+      if (c_face_nodes<DIM, ORDER>(fm) == k) slot_s[k * S::NF + n++] = (int16_t)fm;
+    for (; n < S::NF; ++n) slot_s[k * S::NF + n] = -1;
+  }
+}
+
 // Volume kernel: gradients, pointwise fluxes, face-node records and the
 // volume part of the divergence.  VISC false: the Euler operator (no
 // gradient pass, F = -F_I).
@@ -330,29 +344,18 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT),
   // operators W_r (gradient and divergence) and LIFT_f (gradient), zero padded
   for (int i = threadIdx.x; i < AWN; i += blockDim.x) {
     const int r = i / (MP * KU), row = (i / KU) % MP, k = i % KU;
-    put_a<R>(aw, AWN, i, (row < NP && k < NP) ? c_ref64[S::OFF_W + (r * NP + row) * NP + k] : 0.0);
+    put_a<R>(aw, AWN, i, (row < NP && k < NP) ? refop(S::OFF_W + (r * NP + row) * NP + k) : 0.0);
   }
   if (VISC)
     for (int i = threadIdx.x; i < ALN; i += blockDim.x) {
       const int f = i / (MP * KL), row = (i / KL) % MP, m = i % KL;
       put_a<R>(al, ALN, i,
-               (row < NP && m < NFP) ? c_ref64[S::OFF_LIFT + row * NFN + f * NFP + m] : 0.0);
+               (row < NP && m < NFP) ? refop(S::OFF_LIFT + row * NFN + f * NFP + m) : 0.0);
     }
   for (int i = threadIdx.x; i < V::W1 + NNODE * GST; i += blockDim.x) w1[i] = R(0);
   for (int i = threadIdx.x; i < NFN; i += blockDim.x) fn_s[i] = c_face_nodes<DIM, ORDER>(i);
   for (int i = threadIdx.x; i < a.nperm * NFP; i += blockDim.x) perm_s[i] = a.perm[i];
-  if (threadIdx.x == 0) {
-    // face slots f * NFP + m of each volume node (-1: none)
-    for (int i = 0; i < NP * NF; ++i) slot_s[i] = -1;
-    for (int fm = 0; fm < NFN; ++fm) {
-      const int k = c_face_nodes<DIM, ORDER>(fm);
-      for (int s = 0; s < NF; ++s)
-        if (slot_s[k * NF + s] < 0) {
-          slot_s[k * NF + s] = (int16_t)fm;
-          break;
-        }
-    }
-  }
+  fill_slots<DIM, ORDER>(slot_s);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gq = lane >> 2, tq = lane & 3;
@@ -809,21 +812,11 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT3), 2)
   const bool sources = MIX && a.add_sources;
   for (int i = threadIdx.x; i < AWN; i += blockDim.x) {
     const int r = i / (MP * KU), row = (i / KU) % MP, k = i % KU;
-    put_a<R>(aw, AWN, i, (row < NP && k < NP) ? c_ref64[S::OFF_W + (r * NP + row) * NP + k] : 0.0);
+    put_a<R>(aw, AWN, i, (row < NP && k < NP) ? refop(S::OFF_W + (r * NP + row) * NP + k) : 0.0);
   }
   for (int i = threadIdx.x; i < NNODE * FST + NS * ENP; i += blockDim.x) gfl[i] = R(0);
   for (int i = threadIdx.x; i < NFN; i += blockDim.x) fn_s[i] = c_face_nodes<DIM, ORDER>(i);
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < NP * NF; ++i) slot_s[i] = -1;
-    for (int fm = 0; fm < NFN; ++fm) {
-      const int k = c_face_nodes<DIM, ORDER>(fm);
-      for (int sl = 0; sl < NF; ++sl)
-        if (slot_s[k * NF + sl] < 0) {
-          slot_s[k * NF + sl] = (int16_t)fm;
-          break;
-        }
-    }
-  }
+  fill_slots<DIM, ORDER>(slot_s);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gq = lane >> 2, tq = lane & 3;
   const int nwarps = blockDim.x >> 5;
@@ -1152,7 +1145,7 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT2),
   const int64_t EN = (int64_t)E * NP;
   for (int i = threadIdx.x; i < MP * KF; i += blockDim.x) {
     const int row = i / KF, k = i % KF;
-    put_a<R>(am, MP * KF, i, (row < NP && k < NFN) ? c_ref64[S::OFF_LIFT + row * NFN + k] : 0.0);
+    put_a<R>(am, MP * KF, i, (row < NP && k < NFN) ? refop(S::OFF_LIFT + row * NFN + k) : 0.0);
   }
   for (int i = threadIdx.x; i < NCOL * KF; i += blockDim.x) bm[i] = R(0);
   for (int i = threadIdx.x; i < NFN; i += blockDim.x) fn_s[i] = c_face_nodes<DIM, ORDER>(i);

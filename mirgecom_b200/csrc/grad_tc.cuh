@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(TcGrad<DIM, ORDER, NS>::NT, 1)
     float* bvl = reinterpret_cast<float*>(smem_raw + C::OFF_BV + C::BV_BYTES);
     for (int i = tid; i < C::NV * KV; i += blockDim.x) {
       const int n = i / KV, k = i % KV, r = n / NP, row = n % NP;
-      const double v = (n < DIM * NP && k < NP) ? c_ref64[S::OFF_W + (r * NP + row) * NP + k] : 0.0;
+      const double v = (n < DIM * NP && k < NP) ? refop(S::OFF_W + (r * NP + row) * NP + k) : 0.0;
       float hi, lo;
       split_tf32(v, hi, lo);
       const int o = canon_off(n, k, C::LBO_V) >> 2;
@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(TcGrad<DIM, ORDER, NS>::NT, 1)
     for (int i = tid; i < C::NL * C::KL; i += blockDim.x) {
       const int n = i / C::KL, k = i % C::KL, f = n / NP, row = n % NP;
       const double v = (n < NF * NP && k < NFN && k / NFP == f)
-                           ? c_ref64[S::OFF_LIFT + row * NFN + k]
+                           ? refop(S::OFF_LIFT + row * NFN + k)
                            : 0.0;
       float hi, lo;
       split_tf32(v, hi, lo);

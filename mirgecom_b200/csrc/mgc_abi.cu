@@ -401,7 +401,7 @@ int mgc_upload_reference_operators(int dim, int order, const double* weak_host,
   const int np = simplex_npts(dim, order);
   const int nf = dim + 1;
   const int nfp = simplex_npts(dim - 1, order);
-  const int n = refops_size(dim, order);
+  const int n = refops_size(dim, order) + refgeo_size(dim);
   std::vector<double> p64(n);
   int o = 0;
   for (int i = 0; i < dim * np * np; ++i) p64[o++] = weak_host[i];
