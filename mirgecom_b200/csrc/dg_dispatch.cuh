@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <cstring>
+#include <vector>
 
 #include "dg_kernels.cuh"
 #include "dg_volume.cuh"
@@ -66,11 +67,28 @@ namespace {
 inline int upload_refops_local(int dim, int order, const double* packed64, const float* packed32,
                                const int* fnodes) {
   const int off = refops_offset(dim, order);
-  const int n = refops_size(dim, order);
+  const int n = refmat_size(dim, order);
   const int foff = fnodes_offset(dim, order);
   const int fn = fnodes_size(dim, order);
   if (off < 0) return MGC_E_UNSUPPORTED;
-  if (cudaMemcpyToSymbol(g_refops, packed64, n * sizeof(double), off * sizeof(double)) != cudaSuccess)
+  // WH (dg_refops.cuh)
+  const int np = simplex_npts(dim, order), nf = dim + 1, nfp = simplex_npts(dim - 1, order);
+  const double* lift = packed64 + dim * np * np;
+  const double* nref = packed64 + n;
+  const double* fsr = nref + nf * dim;
+  std::vector<double> wh(packed64, packed64 + dim * np * np);
+  for (int r = 0; r < dim; ++r)
+    for (int f = 0; f < nf; ++f)
+      for (int m = 0; m < nfp; ++m) {
+        const int k = fnodes[f * nfp + m];
+        for (int i = 0; i < np; ++i)
+          wh[(r * np + i) * np + k] -=
+              0.5 * nref[f * dim + r] * fsr[f] * lift[i * nf * nfp + f * nfp + m];
+      }
+  if (cudaMemcpyToSymbol(g_refops, packed64, n * sizeof(double), off * sizeof(double)) !=
+          cudaSuccess ||
+      cudaMemcpyToSymbol(g_refops, wh.data(), wh.size() * sizeof(double),
+                         (off + n) * sizeof(double)) != cudaSuccess)
     return MGC_E_CUDA;
   const int ng = refgeo_size(dim), goff = refgeo_offset(dim, order);
   if (cudaMemcpyToSymbol(c_refgeo64, packed64 + n, ng * sizeof(double), goff * sizeof(double)) !=
@@ -240,15 +258,16 @@ struct Launch {
     }
     return MGC_OK;
   }
-  // workspace of vol_face: face-node records, node-0 shifts, boundary
-  // records, boundary plus states, each 256-byte aligned
+  // workspace of vol_face: face-node records, node-0 shifts and (float64) node
+  // wave speeds, boundary records, boundary plus states, each 256-byte aligned
   static size_t vol_workspace_parts(int64_t nelem, int64_t nbf, size_t* off_s0,
                                     size_t* off_btrace, size_t* off_bplus) {
     using V = VCfg<R, DIM, ORDER, NS, MIX>;
     auto al = [](size_t b) { return (b + 255) / 256 * 256; };
     const size_t nb = (size_t)(nbf > 0 ? nbf : 1);
     const size_t tr = al((size_t)nelem * V::NFN * V::TW * sizeof(R));
-    const size_t s0 = al((size_t)nelem * V::NF * V::NC * sizeof(R));
+    const size_t s0 = al((size_t)nelem * V::NF * V::NC * sizeof(R)) +
+                      (folds<R>() ? al((size_t)nelem * V::NP * sizeof(R)) : 0);
     const size_t bt = al(nb * V::NFP * V::TW * sizeof(R));
     const size_t bp = al(nb * V::NFP * V::NC * sizeof(R));
     if (off_s0) *off_s0 = tr;

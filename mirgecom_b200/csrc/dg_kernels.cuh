@@ -60,6 +60,7 @@ struct DGArgs {
   // volume/face path
   R* trace;            // [E][NF][NFP][TW] face-node records: F.n, lambda, p, c, gamma
   R* s0;               // [E][NF][NC] node-0 flux . n per face (element-constant shift)
+  R* lam;              // [E][NP] node wave speed |v| + c (folds<R>() only)
   R* btrace;           // [nbf][NFP][TW] exterior records of boundary faces
   R* bplus;            // [NC][nbf][NFP] exterior q of the inviscid flux at boundary faces
   const uint8_t* fslot;  // [nperm][NFP] neighbour face slot fn * NFP + m'
@@ -450,14 +451,15 @@ __global__ void __launch_bounds__(256) k_mixture_state_mixed(
 // {{{ gradient kernel
 
 // Gradient pass (grad_cv_operator + grad_t_operator): a persistent kernel
-// that builds W_r and LIFT_f once per CTA and loops over element tiles:
+// that builds WH_r and LIFT_f once per CTA and loops over element tiles:
 //   phase 1  U = u - u0 per node (u0 the element's node-0 value; the discrete
 //            gradient of a constant vanishes, so the shift keeps large means
 //            out of the contraction and changes nothing in exact arithmetic)
 //   phase 2  S = fscale (u* - u0) per face node and group of four fields,
 //            u* the BR1 central value, the prescribed exterior value, or the
-//            interior value (dummy boundary)
-//   phase 3  du_r = W_r U, L_f = LIFT_f S on the tensor cores per (n-tile,
+//            interior value (dummy boundary), less the own half (u- - u0) / 2
+//            that WH carries: an interior face reads the neighbour only
+//   phase 3  du_r = WH_r U, L_f = LIFT_f S on the tensor cores per (n-tile,
 //            m-tile), grad_j = sum_f n_fj L_f - sum_r (dr_r/dx_j) du_r
 template <class R, int DIM, int ORDER, int NS, bool MIX>
 __global__ void __launch_bounds__(256, (Cfg<R, DIM, ORDER, NS, MIX>::MINB_GRAD))
@@ -492,7 +494,7 @@ __global__ void __launch_bounds__(256, (Cfg<R, DIM, ORDER, NS, MIX>::MINB_GRAD))
   // reference operators (zero padded; hi/lo tf32 split on the mixed path)
   for (int i = threadIdx.x; i < AWN; i += blockDim.x) {
     const int r = i / (MP * KU), row = (i / KU) % MP, k = i % KU;
-    put_a<R>(aw, AWN, i, (row < NP && k < NP) ? refop(S::OFF_W + (r * NP + row) * NP + k) : 0.0);
+    put_a<R>(aw, AWN, i, (row < NP && k < NP) ? refop(S::OFF_WH + (r * NP + row) * NP + k) : 0.0);
   }
   for (int i = threadIdx.x; i < ALN; i += blockDim.x) {
     const int f = i / (MP * KL), row = (i / KL) % MP, m = i % KL;
@@ -602,7 +604,8 @@ __global__ void __launch_bounds__(256, (Cfg<R, DIM, ORDER, NS, MIX>::MINB_GRAD))
       R* bcol = bs + e * KS + f * NFPK + m;
       if (mode == 2) {
 #pragma unroll
-        for (int c = 0; c < NU; ++c) bcol[c * EPB * KS] = fsc * bu[(c * EPB + e) * KU + k];
+        for (int c = 0; c < NU; ++c)
+          bcol[c * EPB * KS] = (fsc * R(0.5)) * bu[(c * EPB + e) * KU + k];
         continue;
       }
       const int64_t bstride = (int64_t)a.nbf * NFP, bo = (int64_t)bf * NFP + m;
@@ -624,9 +627,9 @@ __global__ void __launch_bounds__(256, (Cfg<R, DIM, ORDER, NS, MIX>::MINB_GRAD))
       }
 #pragma unroll
       for (int c = 0; c < NU; ++c) {
-        const R um = bu[(c * EPB + e) * KU + k];           // u- - u0
-        const R u0 = u0_s[c * EPB + e];
-        const R v = (mode == 0) ? ((up[c] - u0) + um) * R(0.5) : up[c] - u0;
+        const R du = up[c] - u0_s[c * EPB + e];
+        R v = du * R(0.5);
+        if (mode != 0) v = du - bu[(c * EPB + e) * KU + k] * R(0.5);
         bcol[c * EPB * KS] = fsc * v;
       }
     }
@@ -1225,10 +1228,11 @@ __device__ __forceinline__ void load_group(const R* __restrict__ src, int v0, in
 // (F* = central(F_V) - numflux(F_I)), boundary.py:141-146 (prescribed: the
 // exterior state with the interior gradients) and boundary.py:1027-1049
 // (dummy: the interior flux).  Writes S_c = fsc (F*_c - F0_c . n) for every
-// field c to bcol[c * cstride].  Out of line (arguments by value, no
+// field c to bcol[c * cstride]; with FOLD less the own half (F- - F0) . n / 2
+// that the folded volume operator WH carries.  Out of line (arguments by value, no
 // address of a caller variable taken), so that its face states do not enter
 // the register allocation of the interior fast path.
-template <class R, int DIM, int NP, int NFP, int NS, bool MIX, bool VISC>
+template <class R, int DIM, int NP, int NFP, int NS, bool MIX, bool VISC, bool FOLD>
 __device__ __noinline__ void surface_face_general(const DGArgs<R> a, const GasParams g,
                                                   int64_t EN, int64_t gm, int64_t g0, int m,
                                                   int cn, R n0, R n1, R n2, R fsc,
@@ -1321,7 +1325,8 @@ __device__ __noinline__ void surface_face_general(const DGArgs<R> a, const GasPa
   }
   if (mode == 1) {
 #pragma unroll
-    for (int c = 0; c < NC; ++c) bcol[c * cstride] = fsc * (ftm[c] - f0n[c]);
+    for (int c = 0; c < NC; ++c)
+      bcol[c * cstride] = (FOLD ? R(0.5) * fsc : fsc) * (ftm[c] - f0n[c]);
   } else {
     // F_V . n = F . n + F_I . n on each side
     R fi[NC], fim[NC], fip[NC];
@@ -1332,7 +1337,7 @@ __device__ __noinline__ void surface_face_general(const DGArgs<R> a, const GasPa
     for (int c = 0; c < NC; ++c) {
       R out = -fi[c];
       if (VISC) out += ((ftm[c] + fim[c]) + (fpn[c] + fip[c])) * R(0.5);
-      bcol[c * cstride] = fsc * (out - f0n[c]);
+      bcol[c * cstride] = fsc * (FOLD ? out - (ftm[c] + f0n[c]) * R(0.5) : out - f0n[c]);
     }
   }
 }
@@ -1347,11 +1352,13 @@ __device__ __noinline__ void surface_face_general(const DGArgs<R> a, const GasPa
 //           total flux F = F_V - F_I on both sides, so
 //               F*_V - F*_I = (F^- + F^+) . n / 2 - lambda (q^- - q^+) / 2
 //           (lambda = max(|v| + c) for Rusanov, the node wave speeds the
-//           records carry; 0 for central): no face state is rebuilt.  Other
+//           records carry; 0 for central): no face state is rebuilt, and in
+//           float64 the own half F^- . n / 2 sits in the volume operator WH,
+//           so the neighbour's flux is the only one read.  Other
 //           faces take surface_face_general.  The tile's face pairing is
 //           read from shared memory, so the neighbour gathers start one
 //           global round trip earlier.
-//   lift    rhs = [-W | LIFT] [G ; S] on the tensor cores, one (n-tile,
+//   lift    rhs = [-W(H) | LIFT] [G ; S] on the tensor cores, one (n-tile,
 //           m-tile) per warp work item, plus the species sources.
 // F0 is the record of the element's node 0: subtracting an element-constant
 // flux from every volume and face value leaves the discrete divergence
@@ -1388,7 +1395,7 @@ __global__ void __launch_bounds__(256, (Cfg<R, DIM, ORDER, NS, MIX>::MINB_SURF))
     if (row < NP && k < KR) {
       if (k < DIM * NP) {
         const int r = k / NP, kk = k % NP;
-        v = -refop(S::OFF_W + (r * NP + row) * NP + kk);
+        v = -refop(S::template OFF_WDIV<R> + (r * NP + row) * NP + kk);
       } else {
         v = refop(S::OFF_LIFT + row * NFN + (k - DIM * NP));
       }
@@ -1464,34 +1471,41 @@ __global__ void __launch_bounds__(256, (Cfg<R, DIM, ORDER, NS, MIX>::MINB_SURF))
 #pragma unroll 1
         for (int grp = 0; grp < NG; ++grp) {
           R fmv[GV], fpv[GV], f0v[GV];
-          load_group<R, GV>(a.fbuf + gm * FW, grp * GV, LIM, fmv);
+          if constexpr (!folds<R>()) load_group<R, GV>(a.fbuf + gm * FW, grp * GV, LIM, fmv);
           load_group<R, GV>(a.fbuf + gi * FW, grp * GV, LIM, fpv);
           load_group<R, GV>(a.fbuf + g0 * FW, grp * GV, LIM, f0v);
 #pragma unroll
           for (int cc = 0; cc < CG; ++cc) {
             const int c = grp * CG + cc;
             if (c >= NC) break;
-            R sm_ = R(0), sp_ = R(0), s0 = R(0);
-#pragma unroll
-            for (int j = 0; j < DIM; ++j) {
-              sm_ += fmv[cc * DIM + j] * n[j];
-              sp_ += fpv[cc * DIM + j] * n[j];
-              s0 += f0v[cc * DIM + j] * n[j];
-            }
             const R dq = a.q[c * EN + gm] - a.q[c * EN + gi];
-            const R out = (sm_ + sp_) * R(0.5) - lam * dq * R(0.5);
-            bcol[c * EPB * KB] = fsc * (out - s0);
+            if constexpr (folds<R>()) {
+              R ds = R(0);
+#pragma unroll
+              for (int j = 0; j < DIM; ++j) ds += (fpv[cc * DIM + j] - f0v[cc * DIM + j]) * n[j];
+              bcol[c * EPB * KB] = fsc * ((ds - lam * dq) * R(0.5));
+            } else {
+              R sm_ = R(0), sp_ = R(0), s0 = R(0);
+#pragma unroll
+              for (int j = 0; j < DIM; ++j) {
+                sm_ += fmv[cc * DIM + j] * n[j];
+                sp_ += fpv[cc * DIM + j] * n[j];
+                s0 += f0v[cc * DIM + j] * n[j];
+              }
+              const R out = (sm_ + sp_) * R(0.5) - lam * dq * R(0.5);
+              bcol[c * EPB * KB] = fsc * (out - s0);
+            }
           }
         }
       } else {
-        surface_face_general<R, DIM, NP, NFP, NS, MIX, VISC>(
+        surface_face_general<R, DIM, NP, NFP, NS, MIX, VISC, folds<R>()>(
             a, g, EN, gm, g0, m, cn, n[0], n[1], DIM > 2 ? n[DIM - 1] : R(0), fsc, perm_s,
             bcol, EPB * KB);
       }
     }
     __syncthreads();
 
-    // rhs = [-W | LIFT] [G ; S] on the tensor cores (+ sources).  float32:
+    // rhs = [-W(H) | LIFT] [G ; S] on the tensor cores (+ sources).  float32:
     // one warp item per group of NTG n-tiles and every m-tile, each B value
     // split into its tf32 hi/lo words once; float64: one m-tile and NTG
     // n-tiles per item, so each A fragment load serves NTG products

@@ -14,13 +14,15 @@
 //              F0.n per face (the element-constant shift) into HBM; at
 //              prescribed boundary faces the exterior state's record
 //   volume     rhs = -sum_r W_r (G_r - G0_r) + sources on the tensor cores,
-//              written to HBM
+//              written to HBM (float64: WH_r, the weak derivative with the
+//              element's own half of the central face flux folded in,
+//              dg_refops.cuh)
 // k_face (persistent as well):
-//   faces      per face node: the two records of the face (own, and the
-//              neighbour's through the face pairing), q on both sides, and
-//              the numerical flux F*_V - F*_I (Rusanov / central from the
-//              records alone, HLL through the general path) minus F0.n,
-//              scaled by the face factor
+//   faces      per face node: the neighbour's record (through the face
+//              pairing) and the own one (float64: its wave speed only, WH
+//              having added the own half), q on both sides, and the numerical
+//              flux F*_V - F*_I (Rusanov / central from the records alone, HLL
+//              through the general path) minus F0.n, scaled by the face factor
 //   lift       rhs += LIFT S on the tensor cores
 //
 // Against the three-pass split (gradients, per-node flux records, surface)
@@ -29,7 +31,7 @@
 // contraction (K = Nf * Nfp).  Subtracting the element-constant flux F0 from
 // the volume terms (volume kernel) and from the face terms (face kernel)
 // leaves the discrete divergence unchanged: -W c + LIFT (c.n) = 0 for a
-// constant c.
+// constant c, so -WH c + LIFT (c.n) / 2 = 0.
 #pragma once
 #include "boundary.cuh"
 #include "dg_kernels.cuh"
@@ -341,10 +343,10 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT),
       ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.t_op)) & 15) == 0 &&
       (KU * sizeof(R)) % 16 == 0;
 
-  // operators W_r (gradient and divergence) and LIFT_f (gradient), zero padded
+  // operators W(H)_r (gradient and divergence) and LIFT_f (gradient), zero padded
   for (int i = threadIdx.x; i < AWN; i += blockDim.x) {
     const int r = i / (MP * KU), row = (i / KU) % MP, k = i % KU;
-    put_a<R>(aw, AWN, i, (row < NP && k < NP) ? refop(S::OFF_W + (r * NP + row) * NP + k) : 0.0);
+    put_a<R>(aw, AWN, i, (row < NP && k < NP) ? refop(S::template OFF_WDIV<R> + (r * NP + row) * NP + k) : 0.0);
   }
   if (VISC)
     for (int i = threadIdx.x; i < ALN; i += blockDim.x) {
@@ -454,7 +456,8 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT),
         R* bcol = bs + e * KS + f * NFPK + m;
         if (mode == 2) {
 #pragma unroll
-          for (int c = 0; c < NU; ++c) bcol[c * EPB * KS] = fsc * bu[(c * EPB + e) * KU + k];
+          for (int c = 0; c < NU; ++c)
+            bcol[c * EPB * KS] = (folds<R>() ? fsc * R(0.5) : fsc) * bu[(c * EPB + e) * KU + k];
           continue;
         }
         const int64_t bstride = (int64_t)a.nbf * NFP, bo = (int64_t)bf * NFP + m;
@@ -477,8 +480,12 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT),
 #pragma unroll
         for (int c = 0; c < NU; ++c) {
           const R um = bu[(c * EPB + e) * KU + k];
-          const R u0 = u0_s[c * EPB + e];
-          const R v = (mode == 0) ? ((up[c] - u0) + um) * R(0.5) : up[c] - u0;
+          const R du = up[c] - u0_s[c * EPB + e];
+          R v;
+          if constexpr (folds<R>())
+            v = (mode == 0) ? du * R(0.5) : du - um * R(0.5);
+          else
+            v = (mode == 0) ? (du + um) * R(0.5) : du;
           bcol[c * EPB * KS] = fsc * v;
         }
       }
@@ -636,6 +643,7 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT),
 #pragma unroll
       for (int j = 0; j < DIM; ++j) v2 += st.v[j] * st.v[j];
       const R lam = sqrt(v2) + st.c;
+      if constexpr (folds<R>()) a.lam[gnd] = lam;
       // one record per face slot of this node
 #pragma unroll 1
       for (int sl = 0; sl < NF; ++sl) {
@@ -812,7 +820,7 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT3), 2)
   const bool sources = MIX && a.add_sources;
   for (int i = threadIdx.x; i < AWN; i += blockDim.x) {
     const int r = i / (MP * KU), row = (i / KU) % MP, k = i % KU;
-    put_a<R>(aw, AWN, i, (row < NP && k < NP) ? refop(S::OFF_W + (r * NP + row) * NP + k) : 0.0);
+    put_a<R>(aw, AWN, i, (row < NP && k < NP) ? refop(S::template OFF_WDIV<R> + (r * NP + row) * NP + k) : 0.0);
   }
   for (int i = threadIdx.x; i < NNODE * FST + NS * ENP; i += blockDim.x) gfl[i] = R(0);
   for (int i = threadIdx.x; i < NFN; i += blockDim.x) fn_s[i] = c_face_nodes<DIM, ORDER>(i);
@@ -883,6 +891,7 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT3), 2)
 #pragma unroll
       for (int j = 0; j < DIM; ++j) v2 += st.v[j] * st.v[j];
       const R lam = sqrt(v2) + st.c;
+      if constexpr (folds<R>()) a.lam[gnd] = lam;
 #pragma unroll 1
       for (int sl = 0; sl < NF; ++sl) {
         const int fm = slot_s[k * NF + sl];
@@ -1115,7 +1124,8 @@ __device__ __noinline__ void face_flux_general(const DGArgs<R> a, int64_t EN, in
     R out = -fi[c];
     // F_V . n = F . n + F_I . n on each side; the neighbour record holds -F . n
     if (VISC) out += ((recm[c] + fim[c]) + (-recp[c] + fip[c])) * R(0.5);
-    bcol[c * cstride] = fsc * (out - s0[c]);
+    // less the shift and the own half that WH carries
+    bcol[c * cstride] = fsc * (folds<R>() ? out - (recm[c] + s0[c]) * R(0.5) : out - s0[c]);
   }
 }
 
@@ -1217,7 +1227,8 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT2),
       if (mode == 2) {
         // DummyBoundary: F* = F(q-) . n (boundary.py:1027-1049)
 #pragma unroll
-        for (int c = 0; c < NC; ++c) bcol[c * EPB * KF] = fsc * (recm[c] - s0[c]);
+        for (int c = 0; c < NC; ++c)
+          bcol[c * EPB * KF] = (folds<R>() ? fsc * R(0.5) : fsc) * (recm[c] - s0[c]);
         continue;
       }
       if (a.flux_kind == FLUX_HLL) {
@@ -1228,8 +1239,9 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT2),
         continue;
       }
       R rm[TW], rp[TW];
-      load_record<R, TW>(recm, rm);
+      if constexpr (!folds<R>()) load_record<R, TW>(recm, rm);
       load_record<R, TW>(recp, rp);
+      const R lamm = folds<R>() ? a.lam[gm] : rm[NC];
       R qm[NC], qp[NC], sh[NC];
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
@@ -1237,11 +1249,19 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT2),
         qp[c] = qp_g[c * qstride];
         sh[c] = s0[c];
       }
-      const R lam = (a.flux_kind == FLUX_RUSANOV) ? fmax(rm[NC], rp[NC]) : R(0);
+      const R lam = (a.flux_kind == FLUX_RUSANOV) ? fmax(lamm, rp[NC]) : R(0);
+      if constexpr (folds<R>()) {
+        // F* . n - F0 . n less the own half (F- - F0) . n / 2 that WH carries
+        const R hf = fsc * R(-0.5);
 #pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        const R out = (rm[c] - rp[c]) * R(0.5) - lam * (qm[c] - qp[c]) * R(0.5);
-        bcol[c * EPB * KF] = fsc * (out - sh[c]);
+        for (int c = 0; c < NC; ++c)
+          bcol[c * EPB * KF] = hf * ((rp[c] + sh[c]) + lam * (qm[c] - qp[c]));
+      } else {
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          const R out = (rm[c] - rp[c]) * R(0.5) - lam * (qm[c] - qp[c]) * R(0.5);
+          bcol[c * EPB * KF] = fsc * (out - sh[c]);
+        }
       }
     }
     __syncthreads();

@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(256, 2) k_hex_surface(DGArgs<R> a, GasParams g
           }
         }
       } else {
-        surface_face_general<R, DIM, NP, NFP, NS, MIX, VISC>(a, g, EN, gm, g0, m, cn, n[0], n[1],
+        surface_face_general<R, DIM, NP, NFP, NS, MIX, VISC, false>(a, g, EN, gm, g0, m, cn, n[0], n[1],
                                                              n[2], fsc, perm_s, bcol, NFN);
       }
     }

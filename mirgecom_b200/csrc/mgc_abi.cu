@@ -282,6 +282,10 @@ int operator_impl(int visc, const mgc_mesh_t* mesh, const mgc_gas_t* gas, const 
   char* ws = static_cast<char*>(workspace);
   a.trace = reinterpret_cast<R*>(ws);
   a.s0 = reinterpret_cast<R*>(ws + off_s0);
+  // the node wave speeds (read in float64) follow the shifts, 256-byte aligned
+  const size_t s0_bytes = (size_t)mesh->nelem * (mesh->dim + 1) *
+                          (mesh->dim + 2 + gas->nspecies) * sizeof(R);
+  a.lam = reinterpret_cast<R*>(ws + off_s0 + (s0_bytes + 255) / 256 * 256);
   a.btrace = reinterpret_cast<R*>(ws + off_bt);
   a.bplus = reinterpret_cast<R*>(ws + off_bp);
   a.fslot = mesh->fslot;
@@ -401,7 +405,7 @@ int mgc_upload_reference_operators(int dim, int order, const double* weak_host,
   const int np = simplex_npts(dim, order);
   const int nf = dim + 1;
   const int nfp = simplex_npts(dim - 1, order);
-  const int n = refops_size(dim, order) + refgeo_size(dim);
+  const int n = refmat_size(dim, order) + refgeo_size(dim);
   std::vector<double> p64(n);
   int o = 0;
   for (int i = 0; i < dim * np * np; ++i) p64[o++] = weak_host[i];
