@@ -1,105 +1,63 @@
 // BR1 gradient pass on the 5th-generation tensor cores (tcgen05, TMEM).
 //
-// The same arithmetic as k_grad (dg_kernels.cuh) -- the weak-form gradient
-//   grad_j u = sum_f n_fj LIFT_f (fscale_f u*_f) - sum_r rx_rj W_r u
-// of every conserved field and the temperature, with the element-constant
-// shift u - u_0 and the TF32 three-term split A_hi B_hi + A_hi B_lo +
-// A_lo B_hi -- organised as a warp-specialised pipeline over tiles of
-// EPB elements (grad_operator, mirgecom/navierstokes.py:443-446, and
-// grad_facial_flux, mirgecom/gradient.py):
+// The same gradient as k_grad (dg_kernels.cuh), of every conserved field and
+// the temperature, with the element-constant shift u - u_0 and the TF32
+// three-term split A_hi B_hi + A_hi B_lo + A_lo B_hi (grad_operator,
+// mirgecom/navierstokes.py:443-446, and grad_facial_flux,
+// mirgecom/gradient.py).  On an affine element n_fj fscale_f is
+// sum_r (dr_r/dx_j) c_fr with c_fr = NREF[f][r] FSR[f] (dg_refops.cuh), so the
+// lift needs no per-face products: with reference matrices alone
+//   D_r    = -WH_r (u - u_0) + sum_f (c_fr LIFT_f) P_f
+//   grad_j = sum_r (dr_r/dx_j) D_r,       P_f = u*_f - u_0 - (u-_f - u_0) / 2
+// (P = (u+ - u_0) / 2 on interior faces).  That is DIM accumulator columns per
+// node instead of DIM + NF, 9 multiply-adds per node and field in the epilogue
+// instead of 21, no normals, no face scale and no own face values on interior
+// faces.  The work is a warp-specialised pipeline over tiles of EPB elements:
 //
-//   producer warps 0-11  load the tile's rows of q and T (shifted by their
-//                        first node), the face values fscale (u* - u_0) of
-//                        the neighbours or the boundary, and the element
-//                        geometry; they write the hi/lo copies of the A
-//                        operand [row = (field, element)][k] into one of two
-//                        shared-memory stages and arrive on full[s]; after
-//                        the next tile barrier the group's last thread waits
-//                        on full[s] (complete by then), issues the tcgen05.mma
-//                        products
-//                        D[row][(r, i)] = sum_k U[row][k] W_r[i][k]  (k nodes)
-//                        D[row][(f, i)] = sum_k S[row][k] LIFT_f[i][k]
-//                        into TMEM buffer s and commits to done[s]
+//   producer warps 0-11  shift and split the tile's rows of q and T and the
+//                        face values P into the hi/lo copies of the A operand
+//                        [row = (field, element)][k = node | face node] in one
+//                        of two shared-memory stages and arrive on full[s].
+//                        Each value's registers are loaded again for the NEXT
+//                        tile as soon as they are stored (its face pairing is
+//                        staged two tiles ahead), so the gathers' latency runs
+//                        under the rest of this tile's work.  After the next
+//                        tile's barrier the last thread issues the products
+//                        D[row][(r, i)] = sum_k A[row][k] B[(r, i)][k] into
+//                        TMEM buffer s and commits to done[s]
 //   epilogue warps 12-15 wait on done[s], read their TMEM lanes (one row per
-//                        thread), combine with the metric terms and normals,
-//                        store the gradients and arrive on empty[s]
+//                        thread), combine with the metric terms, store the
+//                        gradients and arrive on empty[s]
 //
-// so the loads of tile i+1 overlap the products and the epilogue of tile i.
+// Tiles: NMT row blocks of 128 (MMA M) with EPM elements each, chosen so that
+// the producers have one face node each: 9 order-3, 16 order-2, 32 order-1
+// tetrahedra of the 7-species mixture.  With the smaller orders in single
+// blocks of 9 elements the barriers and waits of a tile cost as much as the
+// work in it.
+//
+// Bound: the producers' gathers, latency and L1 wavefronts (the products are
+// 0.4 us of a 2.9 us tile).  Against the version with per-face lift columns
+// and no reload in place (CUDA events): order 3, 64^3 cells 4.38 -> 4.33 ms
+// (32^3: 232 M -> 160 M warp instructions), 1260 tetrahedra 17.2 -> 12.4 us;
+// order 2, 40^3 cells 745 us (799 us by k_grad, which it replaces there).
+//
 // Operands use the K-major, non-swizzled canonical layout of the UMMA
 // descriptors: 8-row x 16-byte core matrices, row groups SBO = 128 bytes
-// apart, k chunks LBO bytes apart.  Every mbarrier wait is bounded: after
-// kWaitNs the waiting role sets ST_WAIT_TIMEOUT in the status word and an
-// abort flag that ends the other roles' loops; the kernel then releases its
-// TMEM and returns.
+// apart, k chunks LBO bytes apart; LBO is padded by 16 bytes so that a warp
+// storing 32 consecutive k of one row hits distinct banks.  Every mbarrier
+// wait is bounded: after kWaitNs the waiting role sets ST_WAIT_TIMEOUT in the
+// status word and an abort flag that ends the other roles' loops; the kernel
+// then releases its TMEM and returns.
 #pragma once
 #include <cstdint>
 
+#include "async_copy.cuh"
 #include "dg_kernels.cuh"
 
 namespace mgc {
 
-// {{{ tcgen05 / mbarrier primitives
+// {{{ tcgen05 primitives
 
-__device__ __forceinline__ uint32_t smem_addr(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(uint64_t* b, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(b)), "r"(count)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* b) {
-  asm volatile(
-      "{\n\t.reg .b64 st;\n\tmbarrier.arrive.release.cta.shared::cta.b64 st, [%0];\n\t}" ::"r"(
-          smem_addr(b))
-      : "memory");
-}
-// one test of the phase, the thread suspended until it completes or for at
-// most kSuspendNs
-constexpr uint32_t kSuspendNs = 200000;
-__device__ __forceinline__ bool mbar_try(uint32_t addr, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2, %3;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(addr), "r"(parity), "n"(kSuspendNs)
-      : "memory");
-  return ok != 0;
-}
-// one test of the phase without suspending
-__device__ __forceinline__ bool mbar_test(uint32_t addr, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(addr), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ uint64_t global_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-// a waiting role gives up after this long (the whole kernel normally takes
-// milliseconds)
-constexpr uint64_t kWaitNs = 2000000000ull;
-// Bounded wait for the completion of phase *parity* of barrier *b*; false
-// when the time limit ran out or another role raised *abort* (if given).
-__device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity,
-                                          const volatile int* abort) {
-  const uint32_t a = smem_addr(b);
-  if (mbar_try(a, parity)) return true;
-  const uint64_t t0 = global_ns();
-  for (;;) {
-    if (mbar_try(a, parity)) return true;
-    if (abort && *abort) return false;
-    if (global_ns() - t0 > kWaitNs) return false;
-  }
-}
 __device__ __forceinline__ void fence_async_shared() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
@@ -149,20 +107,23 @@ __device__ __forceinline__ void tc_commit(uint64_t* b) {
           smem_addr(b))
       : "memory");
 }
-// four consecutive 32-bit TMEM columns of this thread's lane
-__device__ __forceinline__ void tc_ld4(uint32_t taddr, uint32_t (&v)[4]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
-               : "r"(taddr));
+// sixteen consecutive 32-bit TMEM columns of this thread's lane
+__device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t* v) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, "
+      "%11, %12, %13, %14, %15}, [%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+        "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
+        "=r"(v[14]), "=r"(v[15])
+      : "r"(taddr));
 }
 // wait for this thread's TMEM loads; the registers are tied to the wait so
 // that no use is scheduled before it
 template <int N>
-__device__ __forceinline__ void tc_wait_ld(uint32_t (&v)[N][4]) {
+__device__ __forceinline__ void tc_wait_ld(uint32_t (&v)[N]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-  for (int i = 0; i < N; ++i)
-    asm volatile("" : "+r"(v[i][0]), "+r"(v[i][1]), "+r"(v[i][2]), "+r"(v[i][3]));
+  for (int i = 0; i < N; ++i) asm volatile("" : "+r"(v[i]));
 }
 
 // }}}
@@ -175,73 +136,57 @@ struct TcGrad {
   static constexpr int NP = S::NP, NF = S::NF, NFP = S::NFP, NFN = NF * NFP;
   static constexpr int NC = DIM + 2 + NS, NU = NC + 1;
   static constexpr int ROWS = 128;                    // MMA M: rows (field, element)
-  static constexpr int EPB = ROWS / NU;               // elements per tile
-  static constexpr int KV = round_up(NP, 8);          // k extent of the volume product
-  static constexpr int KL = round_up(NFN, 8);         // k extent of the lift product
-  static constexpr int KA = KV + KL;                  // A operand k extent
-  static constexpr int NV = round_up(DIM * NP, 16);   // N of the volume product
-  static constexpr int NL = round_up(NF * NP, 16);    // N of the lift product
-  static constexpr int NACC = NV + NL;                // TMEM columns per buffer
-  static constexpr int TCOLS = 512;                   // allocated TMEM columns (2 buffers)
-  static constexpr int BUF_COLS = 256;
+  // twelve producer warps, four epilogue warps
+  static constexpr int GT = 12 * 32, NEPI = 128, NT = GT + NEPI;
+  // row blocks per tile and elements per block: one face node per producer
+  static constexpr int NMT = ORDER == 1 ? 4 : ORDER == 2 ? 2 : 1;
+  static constexpr int EPM = imin(ROWS / NU, GT / (NFN * NMT));
+  static constexpr int EPB = NMT * EPM;
+  static constexpr int KV = round_up(NP, 8);          // k extent of the volume part
+  static constexpr int KA = KV + round_up(NFN, 8);    // k extent with the face values
+  static constexpr int NV = round_up(DIM * NP, 16);   // N: columns (r, i)
+  static constexpr int BUF_COLS = NMT * NV;           // TMEM columns per buffer
+  static constexpr int TCOLS = 2 * BUF_COLS;
   // byte strides of the canonical layouts
   static constexpr int SBO = 128;
-  static constexpr int LBO_A = ROWS / 8 * 128;
-  static constexpr int LBO_V = NV / 8 * 128;
-  static constexpr int LBO_L = NL / 8 * 128;
-  static constexpr int A_BYTES = KA / 4 * LBO_A;      // one copy (hi or lo) of one stage
-  static constexpr int BV_BYTES = KV / 4 * LBO_V;
-  static constexpr int BL_BYTES = KL / 4 * LBO_L;
-  static constexpr int GEO = DIM * DIM + NF * DIM;    // rx, unit normals per element
-  // one producer group of GW warps filling the block's tiles (tile it into
-  // stage it % 2); four epilogue warps.  A single group is what the
-  // deferred product issue assumes: the previous tile's products are issued
-  // after the next tile's barrier, which waits for the stage of the tile
-  // before (two producer groups, each reusing its own stage, would wait for
-  // their own unissued products)
-  static constexpr int NGRP = 1;
-  static constexpr int GW = 12, GT = GW * 32;
-  static constexpr int NPROD = NGRP * GT, NEPI = 128;
-  // producer work items per tile and the rounds of a group they take
-  static constexpr int ROW_ITEMS = NP / 4 * NU * EPB;
-  static constexpr int FACE_ITEMS = NFN * EPB;
+  static constexpr int LBO_A = ROWS / 8 * 128 + 16;
+  static constexpr int LBO_B = NV / 8 * 128;
+  static constexpr int A_BYTES = round_up(KA / 4 * LBO_A, 128);   // one copy of one row block
+  static constexpr int STAGE = 2 * NMT * A_BYTES;                 // [block][hi, lo]
+  static constexpr int B_BYTES = KA / 4 * LBO_B;                  // one copy
+  // rows move in pieces of VW floats
+  static constexpr int VW = NP % 4 == 0 ? 4 : 2;
+  static constexpr int ROW_ITEMS = NP / VW * NU * EPB;
   static constexpr int ROW_ROUNDS = (ROW_ITEMS + GT - 1) / GT;
-  static constexpr int FACE_ROUNDS = (FACE_ITEMS + GT - 1) / GT;
-  static constexpr int NT = NPROD + NEPI;
-  static constexpr int EPI_WARP0 = NPROD / 32;        // a multiple of 4: warp w reads TMEM
-                                                      // lanes 32 (w % 4) ..
-  // per-tile data of a group's tile: face pairing, rx and unit normals,
-  // face scales, the row shifts u_0 (floats/ints), staged one tile ahead
-  static constexpr int SMALL = EPB * NF + EPB * GEO + EPB * NF + NU * EPB;
+  // per-tile data (4-byte words): face pairing, row shifts u_0, metric rx
+  static constexpr int S_U0 = EPB * NF, S_RX = S_U0 + NU * EPB, SMALL = S_RX + EPB * DIM * DIM;
+  static constexpr int SMALL_ROUNDS = (SMALL + GT - 1) / GT;
   // shared-memory carve-up (bytes)
   static constexpr int OFF_BAR = 0;                   // full[2], done[2], empty[2]
   static constexpr int OFF_TMEM = 48;                 // TMEM base address
   static constexpr int OFF_ABORT = 52;                // any role gave up
-  static constexpr int OFF_PABORT = 64;               // each group's copy of it [NGRP]
-  static constexpr int OFF_A = 1024;                  // [stage][hi, lo]
-  static constexpr int OFF_BV = OFF_A + 4 * A_BYTES;  // [hi, lo]
-  static constexpr int OFF_BL = OFF_BV + 2 * BV_BYTES;
-  static constexpr int OFF_GEO = OFF_BL + 2 * BL_BYTES;          // [stage][EPB][GEO] float
-  static constexpr int OFF_SMALL = OFF_GEO + 2 * EPB * GEO * 4;  // [group][2][SMALL] 4-byte
-  static constexpr int OFF_RAW = round_up(OFF_SMALL + NGRP * 2 * SMALL * 4, 16);
-  // [group][NU * EPB][NP] float
-  static constexpr int OFF_FN = OFF_RAW + NGRP * NU * EPB * NP * 4;  // [NFN] int
-  static constexpr int OFF_PERM = OFF_FN + NFN * 4;               // [nperm][NFP] uint8
+  static constexpr int OFF_PABORT = 56;               // the producers' copy [2]
+  static constexpr int OFF_A = 1024;                  // [stage][block][hi, lo]
+  static constexpr int OFF_B = OFF_A + 2 * STAGE;     // [hi, lo]
+  static constexpr int OFF_GEO = OFF_B + 2 * B_BYTES;              // [stage][EPB][DIM][DIM]
+  static constexpr int OFF_SMALL = OFF_GEO + 2 * EPB * DIM * DIM * 4;  // [3][SMALL]
+  static constexpr int OFF_FN = OFF_SMALL + 3 * SMALL * 4;         // [NFN] int
+  static constexpr int OFF_PERM = OFF_FN + NFN * 4;                // [nperm][NFP] uint8
   static size_t smem_bytes(int nperm) { return (size_t)OFF_PERM + (size_t)nperm * NFP + 16; }
-  // whole rows of NP floats in 16-byte pieces; products within the
-  // instruction shapes; two TMEM buffers; the per-tile data one item per
-  // group thread
-  static constexpr bool OK = (NP % 4 == 0) && EPB >= 1 && EPB * NF + NU * EPB <= GT &&
-                             NV <= 256 && NL <= 256 && NACC <= BUF_COLS &&
+  // rows in whole pieces; products within the instruction shapes; TMEM
+  // allocations are powers of two
+  static constexpr bool OK = NP % 2 == 0 && EPM >= 1 && NFN * EPB <= GT && NV <= 256 &&
+                             (TCOLS == 128 || TCOLS == 256 || TCOLS == 512) &&
                              OFF_PERM + 64 * NFP <= 227 * 1024;
 };
 
-// the benchmark's configuration (order-3 tetrahedra, 7 species) fits
-static_assert(TcGrad<3, 3, 7>::OK, "tcgen05 gradient kernel no longer fits order-3 tets");
+// every order of the reacting mixture on tetrahedra fits
+static_assert(TcGrad<3, 1, 7>::OK && TcGrad<3, 2, 7>::OK && TcGrad<3, 3, 7>::OK,
+              "tcgen05 gradient kernel no longer fits the tetrahedra");
 
 // byte offset of element (row, k) in a canonical K-major no-swizzle operand
 __device__ __forceinline__ int canon_off(int row, int k, int lbo) {
-  return (k >> 2) * lbo + (row >> 3) * 128 + (row & 7) * 16 + (k & 3) * 4;
+  return (k >> 2) * lbo + row * 16 + (k & 3) * 4;    // row groups are 8 * 16 bytes
 }
 
 __device__ __forceinline__ void split_f32(float v, float& hi, float& lo) {
@@ -249,6 +194,29 @@ __device__ __forceinline__ void split_f32(float v, float& hi, float& lo) {
   hi = __uint_as_float(h);
   lo = __uint_as_float(to_tf32(v - hi));
 }
+
+// VW consecutive floats as one vector access
+template <int VW> struct VecF;
+template <> struct VecF<4> {
+  float4 v;
+  __device__ __forceinline__ void load(const float* p) { v = __ldg(reinterpret_cast<const float4*>(p)); }
+  __device__ __forceinline__ void store(float* p) const { *reinterpret_cast<float4*>(p) = v; }
+  __device__ __forceinline__ void shift_split(float u0, VecF& h, VecF& l) const {
+    split_f32(v.x - u0, h.v.x, l.v.x);
+    split_f32(v.y - u0, h.v.y, l.v.y);
+    split_f32(v.z - u0, h.v.z, l.v.z);
+    split_f32(v.w - u0, h.v.w, l.v.w);
+  }
+};
+template <> struct VecF<2> {
+  float2 v;
+  __device__ __forceinline__ void load(const float* p) { v = __ldg(reinterpret_cast<const float2*>(p)); }
+  __device__ __forceinline__ void store(float* p) const { *reinterpret_cast<float2*>(p) = v; }
+  __device__ __forceinline__ void shift_split(float u0, VecF& h, VecF& l) const {
+    split_f32(v.x - u0, h.v.x, l.v.x);
+    split_f32(v.y - u0, h.v.y, l.v.y);
+  }
+};
 
 // }}}
 
@@ -260,8 +228,9 @@ __global__ void __launch_bounds__(TcGrad<DIM, ORDER, NS>::NT, 1)
   using C = TcGrad<DIM, ORDER, NS>;
   using S = Simplex<DIM, ORDER>;
   constexpr int NP = C::NP, NF = C::NF, NFP = C::NFP, NFN = C::NFN, NC = C::NC, NU = C::NU;
-  constexpr int EPB = C::EPB, KV = C::KV, GEO = C::GEO, GT = C::GT;
-  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  constexpr int EPB = C::EPB, EPM = C::EPM, NMT = C::NMT, KV = C::KV, KA = C::KA, NV = C::NV;
+  constexpr int GT = C::GT, VW = C::VW, DD = DIM * DIM;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw + C::OFF_BAR);
   uint64_t* done = full + 2;
   uint64_t* empty = full + 4;
@@ -269,6 +238,7 @@ __global__ void __launch_bounds__(TcGrad<DIM, ORDER, NS>::NT, 1)
   volatile int* abort_s = reinterpret_cast<volatile int*>(smem_raw + C::OFF_ABORT);
   volatile int* pabort_s = reinterpret_cast<volatile int*>(smem_raw + C::OFF_PABORT);
   float* geo_s = reinterpret_cast<float*>(smem_raw + C::OFF_GEO);
+  uint32_t* small_s = reinterpret_cast<uint32_t*>(smem_raw + C::OFF_SMALL);
   int* fn_s = reinterpret_cast<int*>(smem_raw + C::OFF_FN);
   uint8_t* perm_s = smem_raw + C::OFF_PERM;
 
@@ -286,35 +256,31 @@ __global__ void __launch_bounds__(TcGrad<DIM, ORDER, NS>::NT, 1)
       mbar_init(empty + s, C::NEPI);
     }
     *abort_s = 0;
-    for (int i = 0; i < C::NGRP; ++i) pabort_s[i] = 0;
+    pabort_s[0] = pabort_s[1] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   {
     float4* az = reinterpret_cast<float4*>(smem_raw + C::OFF_A);
-    for (int i = tid; i < 4 * C::A_BYTES / 16; i += blockDim.x) az[i] = make_float4(0, 0, 0, 0);
-    float* bvh = reinterpret_cast<float*>(smem_raw + C::OFF_BV);
-    float* bvl = reinterpret_cast<float*>(smem_raw + C::OFF_BV + C::BV_BYTES);
-    for (int i = tid; i < C::NV * KV; i += blockDim.x) {
-      const int n = i / KV, k = i % KV, r = n / NP, row = n % NP;
-      const double v = (n < DIM * NP && k < NP) ? refop(S::OFF_W + (r * NP + row) * NP + k) : 0.0;
+    for (int i = tid; i < 2 * C::STAGE / 16; i += blockDim.x) az[i] = make_float4(0, 0, 0, 0);
+    float* bh = reinterpret_cast<float*>(smem_raw + C::OFF_B);
+    float* bl = reinterpret_cast<float*>(smem_raw + C::OFF_B + C::B_BYTES);
+    for (int i = tid; i < NV * KA; i += blockDim.x) {
+      const int n = i / KA, k = i % KA, r = n / NP, row = n % NP;
+      double v = 0.0;
+      if (n < DIM * NP) {
+        if (k < NP) {
+          v = -refop(S::OFF_WH + (r * NP + row) * NP + k);
+        } else if (k >= KV && k - KV < NFN) {
+          const int f = (k - KV) / NFP;
+          v = RefBank<double>::get(S::OFF_NREF + f * DIM + r) *
+              RefBank<double>::get(S::OFF_FSR + f) * refop(S::OFF_LIFT + row * NFN + k - KV);
+        }
+      }
       float hi, lo;
       split_tf32(v, hi, lo);
-      const int o = canon_off(n, k, C::LBO_V) >> 2;
-      bvh[o] = hi;
-      bvl[o] = lo;
-    }
-    float* blh = reinterpret_cast<float*>(smem_raw + C::OFF_BL);
-    float* bll = reinterpret_cast<float*>(smem_raw + C::OFF_BL + C::BL_BYTES);
-    for (int i = tid; i < C::NL * C::KL; i += blockDim.x) {
-      const int n = i / C::KL, k = i % C::KL, f = n / NP, row = n % NP;
-      const double v = (n < NF * NP && k < NFN && k / NFP == f)
-                           ? refop(S::OFF_LIFT + row * NFN + k)
-                           : 0.0;
-      float hi, lo;
-      split_tf32(v, hi, lo);
-      const int o = canon_off(n, k, C::LBO_L) >> 2;
-      blh[o] = hi;
-      bll[o] = lo;
+      const int o = canon_off(n, k, C::LBO_B) >> 2;
+      bh[o] = hi;
+      bl[o] = lo;
     }
     for (int i = tid; i < NFN; i += blockDim.x) fn_s[i] = c_face_nodes<DIM, ORDER>(i);
     for (int i = tid; i < a.nperm * NFP; i += blockDim.x) perm_s[i] = a.perm[i];
@@ -327,295 +293,98 @@ __global__ void __launch_bounds__(TcGrad<DIM, ORDER, NS>::NT, 1)
   tc_fence_after();
   const uint32_t tmem = *tmem_s;
 
-  if (warp < C::NPROD / 32) {
-    // ================= producers: group grp fills the block's tiles
-    // it = grp, grp + NGRP, ..., tile it into stage it % 2
-    constexpr int RR = C::ROW_ROUNDS, FR = C::FACE_ROUNDS;
-    const int grp = tid / GT, gtid = tid % GT;
-    // group buffers: per-tile data [2][SMALL], shifted rows [NU * EPB][NP]
-    float* small_g = reinterpret_cast<float*>(smem_raw + C::OFF_SMALL) + grp * 2 * C::SMALL;
-    float* raw = reinterpret_cast<float*>(smem_raw + C::OFF_RAW) + grp * NU * EPB * NP;
-    auto conn_of = [&](int b) { return reinterpret_cast<int32_t*>(small_g + b * C::SMALL); };
-    auto geo_of = [&](int b) { return small_g + b * C::SMALL + EPB * NF; };
-    auto fs_of = [&](int b) { return small_g + b * C::SMALL + EPB * NF + EPB * GEO; };
-    auto u0_of = [&](int b) { return small_g + b * C::SMALL + 2 * EPB * NF + EPB * GEO; };
-    // per-tile data of tile *tl*: loads, then (after this tile's work) the
-    // derived values into buffer *b*
-    struct Small {
-      int32_t cn;
-      float rxe[DIM * DIM];
-      float u0;
-      bool gok, uok;
-    };
-    auto small_load = [&](int tl, Small& sm) {
+  if (tid < GT) {
+    // ================= producers
+    constexpr int RR = C::ROW_ROUNDS, SR = C::SMALL_ROUNDS;
+    // this thread's face node: element fe of the tile, face slot ffm
+    const int ffm = tid % NFN, fe = tid / NFN;
+    const int ff = ffm / NFP, fm_ = ffm % NFP;
+    const int fk = fn_s[ffm];
+    auto field = [&](int c) { return c < NC ? a.q + c * EN : a.t_op; };
+    auto small_load = [&](int tl, uint32_t (&w)[SR]) {
       const int e1 = tl * EPB, n1 = imin(EPB, EOWN - e1);
-      const int gi = gtid, ui = gtid - EPB * NF;
-      sm.gok = gi < n1 * NF;
-      sm.uok = ui >= 0 && ui < NU * EPB && ui % EPB < n1;
-      if (sm.gok) {
-        sm.cn = __ldg(a.conn + (int64_t)e1 * NF + gi);
-        const float* rxg = a.rx + (int64_t)(e1 + gi / NF) * DIM * DIM;
 #pragma unroll
-        for (int i = 0; i < DIM * DIM; ++i) sm.rxe[i] = __ldg(rxg + i);
-      }
-      if (sm.uok) {
-        const int c = ui / EPB, e = ui % EPB;
-        sm.u0 = __ldg((c < NC ? a.q + c * EN : a.t_op) + (int64_t)(e1 + e) * NP);
-      }
-    };
-    auto small_store = [&](const Small& sm, int b) {
-      if (sm.gok) {
-        const int gi = gtid, e = gi / NF, f = gi % NF;
-        float* pg = geo_of(b) + e * GEO;
-        conn_of(b)[gi] = sm.cn;
-        float nv[DIM];
-        float mag2 = 0;
-#pragma unroll
-        for (int j = 0; j < DIM; ++j) {
-          float acc = 0;
-#pragma unroll
-          for (int r = 0; r < DIM; ++r)
-            acc += sm.rxe[r * DIM + j] * RefBank<float>::get(S::OFF_NREF + f * DIM + r);
-          nv[j] = acc;
-          mag2 += acc * acc;
-        }
-        const float mag = sqrtf(mag2);
-#pragma unroll
-        // approximate quotient: an IEEE division site (with its out-of-line
-        // slow path) cost this whole kernel 1.1 ms at 80^3; the normals
-        // differ from the other kernels' by a few ulp
-        for (int j = 0; j < DIM; ++j) pg[DIM * DIM + f * DIM + j] = __fdividef(nv[j], mag);
-        fs_of(b)[gi] = mag * RefBank<float>::get(S::OFF_FSR + f);
-        if (f == 0) {
-#pragma unroll
-          for (int i = 0; i < DIM * DIM; ++i) pg[i] = sm.rxe[i];
+      for (int j = 0; j < SR; ++j) {
+        const int i = tid + j * GT;
+        w[j] = 0;
+        if (i < C::S_U0) {
+          if (i / NF < n1) w[j] = (uint32_t)__ldg(a.conn + (int64_t)e1 * NF + i);
+        } else if (i < C::S_RX) {
+          const int e = (i - C::S_U0) % EPB, c = (i - C::S_U0) / EPB;
+          if (e < n1) w[j] = __float_as_uint(__ldg(field(c) + (int64_t)(e1 + e) * NP));
+        } else if (i < C::SMALL) {
+          const int m = i - C::S_RX;
+          if (m / DD < n1) w[j] = __float_as_uint(__ldg(a.rx + (int64_t)e1 * DD + m));
         }
       }
-      if (sm.uok) u0_of(b)[gtid - EPB * NF] = sm.u0;
     };
-    // D[s] = A[s] B^T: the volume products into columns [0, NV), the lift
-    // products into [NV, NV + NL), three split terms per k step
+    auto small_store = [&](const uint32_t (&w)[SR], int b) {
+#pragma unroll
+      for (int j = 0; j < SR; ++j)
+        if (tid + j * GT < C::SMALL) small_s[b * C::SMALL + tid + j * GT] = w[j];
+    };
+    VecF<VW> rv[RR];
+    float nb[NU];
+    int fmode = -1;
+    auto row_load = [&](int tl, int j) {
+      const int idx = tid + j * GT;
+      const int kc = idx % (NP / VW), e = (idx / (NP / VW)) % EPB, c = idx / (NP / VW * EPB);
+      if (idx < C::ROW_ITEMS && tl * EPB + e < EOWN)
+        rv[j].load(field(c) + (int64_t)(tl * EPB + e) * NP + kc * VW);
+    };
+    // mode of this thread's face node in tile tl (pairing words *conn_b*):
+    // -1 none, 0 interior (en, kn its neighbour node), 1 exterior value,
+    // 2 interior value, 3 Mengaldo
+    auto face_mode = [&](int tl, const uint32_t* conn_b, int64_t& gi) {
+      gi = 0;
+      if (tid >= NFN * EPB || tl * EPB + fe >= EOWN) return -1;
+      const int cn = (int)conn_b[fe * NF + ff];
+      if (cn >= 0) {
+        const int en = cn >> 8, pr = cn & 255;
+        const int kn = (pr < a.nperm) ? perm_s[pr * NFP + fm_] : NP;
+        if (en < E && kn < NP) {
+          gi = (int64_t)en * NP + kn;
+          return 0;
+        }
+        atomicOr(a.status, ST_BAD_INDEX);
+        return 2;
+      }
+      const int bf = -(cn + 1);
+      int kind = (bf < a.nbf) ? a.bkind[bf] : -1;
+      if ((bk_needs_bext(kind) && !a.bext) || kind > BK_OUTFLOW) kind = -1;
+      if (kind < 0) atomicOr(a.status, ST_BAD_INDEX);
+      return kind == BK_PRESCRIBED ? 1 : bk_mengaldo(kind) ? 3 : 2;
+    };
+    // D[s] = A[s] B^T, the two correction terms of every k step first: the
+    // accumulator (which truncates) is then near its final size for KA / 8
+    // additions instead of 3 KA / 8
     auto issue_products = [&](int s) {
-      constexpr uint32_t IDV = umma_idesc_tf32(C::ROWS, C::NV);
-      constexpr uint32_t IDL = umma_idesc_tf32(C::ROWS, C::NL);
-      const uint32_t ah = smem_addr(smem_raw + C::OFF_A) + (2 * s) * C::A_BYTES;
-      const uint32_t al = ah + C::A_BYTES;
-      const uint32_t bvh = smem_addr(smem_raw + C::OFF_BV), bvl = bvh + C::BV_BYTES;
-      const uint32_t blh = smem_addr(smem_raw + C::OFF_BL), bll = blh + C::BL_BYTES;
-      const uint32_t d = tmem + (uint32_t)(s * C::BUF_COLS);
+      constexpr uint32_t ID = umma_idesc_tf32(C::ROWS, NV);
+      const uint32_t bh = smem_addr(smem_raw + C::OFF_B), bl = bh + C::B_BYTES;
+#pragma unroll 1
+      for (int mt = 0; mt < NMT; ++mt) {
+        const uint32_t ah = smem_addr(smem_raw + C::OFF_A) + s * C::STAGE + 2 * mt * C::A_BYTES;
+        const uint32_t al = ah + C::A_BYTES;
+        const uint32_t d = tmem + (uint32_t)(s * C::BUF_COLS + mt * NV);
 #pragma unroll
-      for (int ks = 0; ks < KV / 8; ++ks) {
-        const uint32_t ao = 2 * ks * C::LBO_A, bo = 2 * ks * C::LBO_V;
-        tc_mma_tf32(d, umma_desc(al + ao, C::LBO_A, C::SBO), umma_desc(bvh + bo, C::LBO_V, C::SBO),
-                    IDV, ks > 0);
-        tc_mma_tf32(d, umma_desc(ah + ao, C::LBO_A, C::SBO), umma_desc(bvl + bo, C::LBO_V, C::SBO),
-                    IDV, 1);
-        tc_mma_tf32(d, umma_desc(ah + ao, C::LBO_A, C::SBO), umma_desc(bvh + bo, C::LBO_V, C::SBO),
-                    IDV, 1);
-      }
+        for (int ks = 0; ks < KA / 8; ++ks) {
+          const uint32_t ao = 2 * ks * C::LBO_A, bo = 2 * ks * C::LBO_B;
+          tc_mma_tf32(d, umma_desc(al + ao, C::LBO_A, C::SBO),
+                      umma_desc(bh + bo, C::LBO_B, C::SBO), ID, ks > 0);
+          tc_mma_tf32(d, umma_desc(ah + ao, C::LBO_A, C::SBO),
+                      umma_desc(bl + bo, C::LBO_B, C::SBO), ID, 1);
+        }
 #pragma unroll
-      for (int ks = 0; ks < C::KL / 8; ++ks) {
-        const uint32_t ao = (KV / 4 + 2 * ks) * C::LBO_A, bo = 2 * ks * C::LBO_L;
-        const uint32_t dl = d + C::NV;
-        tc_mma_tf32(dl, umma_desc(al + ao, C::LBO_A, C::SBO),
-                    umma_desc(blh + bo, C::LBO_L, C::SBO), IDL, ks > 0);
-        tc_mma_tf32(dl, umma_desc(ah + ao, C::LBO_A, C::SBO),
-                    umma_desc(bll + bo, C::LBO_L, C::SBO), IDL, 1);
-        tc_mma_tf32(dl, umma_desc(ah + ao, C::LBO_A, C::SBO),
-                    umma_desc(blh + bo, C::LBO_L, C::SBO), IDL, 1);
+        for (int ks = 0; ks < KA / 8; ++ks) {
+          const uint32_t ao = 2 * ks * C::LBO_A, bo = 2 * ks * C::LBO_B;
+          tc_mma_tf32(d, umma_desc(ah + ao, C::LBO_A, C::SBO),
+                      umma_desc(bh + bo, C::LBO_B, C::SBO), ID, 1);
+        }
       }
     };
     int issued = 0, last_issued = -1;
     int pending = -1;          // a filled tile whose products are not issued yet
-    const int first = blockIdx.x + grp * (int)gridDim.x;
-    const int step = C::NGRP * (int)gridDim.x;
-    if (first < ntiles) {
-      Small sm0;
-      small_load(first, sm0);
-      small_store(sm0, 0);
-    }
-    for (int u = 0, tile = first; tile < ntiles; ++u, tile += step) {
-      const int b = u & 1;
-      const int it = grp + u * C::NGRP;
-      const int s = it & 1;
-      const uint32_t use = (uint32_t)it >> 1;
-      if (gtid == 0) {
-        bool ok = true;
-        if (use >= 1) ok = mbar_wait(empty + s, (use - 1) & 1, abort_s);
-        if (!ok) {
-          atomicOr(a.status, ST_WAIT_TIMEOUT);
-          *abort_s = 1;
-        }
-        pabort_s[grp] = *abort_s;
-      }
-      // this tile's staged data is complete, the group is done with the
-      // other buffer and with the shifted rows, and stage s is free
-      asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(GT) : "memory");
-      if (pabort_s[grp]) break;
-      // the previous tile's products, issued by the group's last thread (it
-      // has no face item and one row piece at most): its wait and issue
-      // overlap the other threads' loads instead of delaying the barrier
-      if (gtid == GT - 1 && pending >= 0) {
-        const int ps = pending & 1;
-        if (!mbar_wait(full + ps, ((uint32_t)pending >> 1) & 1, abort_s)) {
-          atomicOr(a.status, ST_WAIT_TIMEOUT);
-          *abort_s = 1;
-        } else {
-          tc_fence_after();
-          issue_products(ps);
-          tc_commit(done + ps);
-          ++issued;
-          last_issued = pending;
-        }
-        pending = -1;
-      }
-      const int e0 = tile * EPB;
-      const int ne = imin(EPB, EOWN - e0);
-      const int32_t* conn_b = conn_of(b);
-      const float* fs_b = fs_of(b);
-      const float* u0_b = u0_of(b);
-      const float* pg_b = geo_of(b);
-      unsigned char* ahi = smem_raw + C::OFF_A + (2 * s) * C::A_BYTES;
-      unsigned char* alo = ahi + C::A_BYTES;
-
-      // ---- every global load of this thread's items first: rows of q and T
-      // in 16-byte pieces (item -> piece kc, field c, element e), the
-      // neighbours' values at this thread's face nodes (item -> face node
-      // fm, element e)
-      float4 rv[RR];
-#pragma unroll
-      for (int j = 0; j < RR; ++j) {
-        const int idx = gtid + j * GT;
-        const int e = idx % EPB, c = (idx / EPB) % NU, kc = idx / (EPB * NU);
-        if (idx < C::ROW_ITEMS && e < ne) {
-          const float* src = (c < NC ? a.q + c * EN : a.t_op) + (int64_t)(e0 + e) * NP;
-          rv[j] = __ldg(reinterpret_cast<const float4*>(src) + kc);
-        }
-      }
-      float nb[FR][NU];
-      int fmode[FR];
-#pragma unroll
-      for (int j = 0; j < FR; ++j) {
-        const int idx = gtid + j * GT;
-        const int e = idx % EPB, fm = idx / EPB, f = fm / NFP, m = fm % NFP;
-        fmode[j] = -1;
-        if (idx < C::FACE_ITEMS && e < ne) {
-          const int cn = conn_b[e * NF + f];
-          // 0 two-sided average, 1 exterior value, 2 interior value, 3 Mengaldo
-          int mode = 2;
-          if (cn >= 0) {
-            const int en = cn >> 8, pr = cn & 255;
-            const int kn = (pr < a.nperm) ? perm_s[pr * NFP + m] : NP;
-            if (en >= E || kn >= NP) {
-              atomicOr(a.status, ST_BAD_INDEX);
-            } else {
-              const int64_t gi = (int64_t)en * NP + kn;
-#pragma unroll
-              for (int c = 0; c < NU; ++c)
-                nb[j][c] = __ldg((c < NC ? a.q + c * EN : a.t_op) + gi);
-              mode = 0;
-            }
-          } else {
-            const int bf = -(cn + 1);
-            int kind = (bf < a.nbf) ? a.bkind[bf] : -1;
-            if ((bk_needs_bext(kind) && !a.bext) || kind > BK_OUTFLOW) kind = -1;
-            if (kind == BK_PRESCRIBED) {
-              mode = 1;
-            } else if (bk_mengaldo(kind)) {
-              mode = 3;
-            } else if (kind < 0) {
-              atomicOr(a.status, ST_BAD_INDEX);
-            }
-          }
-          fmode[j] = mode;
-        }
-      }
-      // one group: the next tile's per-tile data loads with this tile's
-      const bool more = tile + step < ntiles;
-      Small sm;
-      sm.gok = sm.uok = false;
-      if (C::NGRP == 1 && more) small_load(tile + step, sm);
-
-      // ---- rows: shift, keep the shifted row, split, store
-#pragma unroll
-      for (int j = 0; j < RR; ++j) {
-        const int idx = gtid + j * GT;
-        const int e = idx % EPB, c = (idx / EPB) % NU, kc = idx / (EPB * NU);
-        if (idx < C::ROW_ITEMS && e < ne) {
-          const float u0 = u0_b[c * EPB + e];
-          const float4 x = make_float4(rv[j].x - u0, rv[j].y - u0, rv[j].z - u0, rv[j].w - u0);
-          *reinterpret_cast<float4*>(raw + (c * EPB + e) * NP + kc * 4) = x;
-          float4 h, l;
-          split_f32(x.x, h.x, l.x);
-          split_f32(x.y, h.y, l.y);
-          split_f32(x.z, h.z, l.z);
-          split_f32(x.w, h.w, l.w);
-          const int o = canon_off(c * EPB + e, kc * 4, C::LBO_A);
-          *reinterpret_cast<float4*>(ahi + o) = h;
-          *reinterpret_cast<float4*>(alo + o) = l;
-        }
-      }
-      // the shifted rows are complete
-      asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(GT) : "memory");
-      // ---- face values fscale * (u* - u0), own values from the shifted rows
-#pragma unroll
-      for (int j = 0; j < FR; ++j) {
-        if (fmode[j] < 0) continue;
-        const int idx = gtid + j * GT;
-        const int e = idx % EPB, fm = idx / EPB, f = fm / NFP, m = fm % NFP;
-        const int k = fn_s[fm];
-        const float fsc = fs_b[e * NF + f];
-        int mode = fmode[j];
-        if (mode == 1 || mode == 3) {
-          const int bf = -(conn_b[e * NF + f] + 1);
-          float up[NU];
-          if (mode == 3) {
-            const float* nf = pg_b + e * GEO + DIM * DIM + f * DIM;
-            mengaldo_grad_value<float, DIM, NS, true>(a, g, a.bkind[bf], bf, m, NFP, EN,
-                                                      (int64_t)(e0 + e) * NP + k, nf[0], nf[1],
-                                                      DIM > 2 ? nf[DIM - 1] : 0.f, up);
-          } else {
-            const int64_t bstride = (int64_t)a.nbf * NFP, bo = (int64_t)bf * NFP + m;
-#pragma unroll
-            for (int c = 0; c < NU; ++c) up[c] = a.bext[c * bstride + bo];
-          }
-#pragma unroll
-          for (int c = 0; c < NU; ++c) nb[j][c] = up[c];
-          mode = 1;
-        }
-        const int kk = KV + fm;
-#pragma unroll
-        for (int c = 0; c < NU; ++c) {
-          const float u0 = u0_b[c * EPB + e];
-          const float um = raw[(c * EPB + e) * NP + k];
-          float v;
-          if (mode == 0)
-            v = ((nb[j][c] - u0) + um) * 0.5f;
-          else if (mode == 1)
-            v = nb[j][c] - u0;
-          else
-            v = um;
-          float hi, lo;
-          split_f32(fsc * v, hi, lo);
-          const int o = canon_off(c * EPB + e, kk, C::LBO_A);
-          *reinterpret_cast<float*>(ahi + o) = hi;
-          *reinterpret_cast<float*>(alo + o) = lo;
-        }
-      }
-      // ---- the epilogue's copy of the geometry; the group's next tile's
-      // data (its latency hidden by the other group's work)
-      float* geo = geo_s + s * EPB * GEO;
-      for (int i = gtid; i < ne * GEO; i += GT) geo[i] = pg_b[i];
-      if (more) {
-        if (C::NGRP > 1) small_load(tile + step, sm);
-        small_store(sm, b ^ 1);
-      }
-      fence_async_shared();
-      mbar_arrive(full + s);
-      if (gtid == GT - 1) pending = it;
-    }
-    // the last tile's products (after a normal end of the loop)
-    if (gtid == GT - 1 && pending >= 0 && !*abort_s) {
+    auto issue_pending = [&]() {
       const int ps = pending & 1;
       if (!mbar_wait(full + ps, ((uint32_t)pending >> 1) & 1, abort_s)) {
         atomicOr(a.status, ST_WAIT_TIMEOUT);
@@ -627,10 +396,147 @@ __global__ void __launch_bounds__(TcGrad<DIM, ORDER, NS>::NT, 1)
         ++issued;
         last_issued = pending;
       }
+      pending = -1;
+    };
+    const int first = blockIdx.x, step = (int)gridDim.x;
+    {
+      // per-tile data of the first two tiles, then the first tile's values
+      uint32_t w[SR];
+      small_load(first, w);
+      small_store(w, 0);
+      if (first + step < ntiles) {
+        small_load(first + step, w);
+        small_store(w, 1);
+      }
+      asm volatile("bar.sync 1, %0;" ::"n"(GT) : "memory");
+#pragma unroll
+      for (int j = 0; j < RR; ++j) row_load(first, j);
+      int64_t gi;
+      fmode = face_mode(first, small_s, gi);
+      if (fmode == 0) {
+#pragma unroll
+        for (int c = 0; c < NU; ++c) nb[c] = __ldg(field(c) + gi);
+      }
     }
+    for (int it = 0, tile = first, b = 0; tile < ntiles; ++it, tile += step) {
+      const int s = it & 1;
+      const uint32_t use = (uint32_t)it >> 1;
+      if (tid == 0) {
+        bool ok = true;
+        if (use >= 1) ok = mbar_wait(empty + s, (use - 1) & 1, abort_s);
+        if (!ok) {
+          atomicOr(a.status, ST_WAIT_TIMEOUT);
+          *abort_s = 1;
+        }
+        pabort_s[s] = *abort_s;
+      }
+      // this tile's and the next one's per-tile data are complete, the
+      // producers are done with the third buffer, and stage s is free
+      asm volatile("bar.sync 1, %0;" ::"n"(GT) : "memory");
+      // (thread 0 may be a tile ahead, never two: its next word is the other one)
+      if (pabort_s[s]) break;
+      // the previous tile's products: their issue overlaps the other
+      // threads' work
+      if (tid == GT - 1 && pending >= 0) issue_pending();
+      const int ne = imin(EPB, EOWN - tile * EPB);
+      const bool more = tile + step < ntiles;
+      const int bn = b == 2 ? 0 : b + 1;
+      const uint32_t* small_b = small_s + b * C::SMALL;
+      const float* u0_b = reinterpret_cast<const float*>(small_b) + C::S_U0;
+      const float* rx_b = reinterpret_cast<const float*>(small_b) + C::S_RX;
+      unsigned char* stage = smem_raw + C::OFF_A + s * C::STAGE;
+      uint32_t w[SR];
+      const bool more2 = tile + 2 * step < ntiles;
+      if (more2) small_load(tile + 2 * step, w);
+
+      // ---- rows: shift, split, store; reload for the next tile
+#pragma unroll
+      for (int j = 0; j < RR; ++j) {
+        const int idx = tid + j * GT;
+        const int kc = idx % (NP / VW), e = (idx / (NP / VW)) % EPB, c = idx / (NP / VW * EPB);
+        if (idx < C::ROW_ITEMS && e < ne) {
+          VecF<VW> h, l;
+          rv[j].shift_split(u0_b[c * EPB + e], h, l);
+          unsigned char* blk = stage + 2 * (e / EPM) * C::A_BYTES;
+          const int o = canon_off(c * EPM + e % EPM, kc * VW, C::LBO_A);
+          h.store(reinterpret_cast<float*>(blk + o));
+          l.store(reinterpret_cast<float*>(blk + C::A_BYTES + o));
+        }
+        if (more) row_load(tile + step, j);
+      }
+
+      // ---- face value P of this thread's face node; reload for the next tile
+      const int mode = fmode;
+      int64_t gn = 0;
+      if (more) fmode = face_mode(tile + step, small_s + bn * C::SMALL, gn);
+      const bool reload = more && fmode == 0;
+      if (mode >= 0) {
+        unsigned char* fdst = stage + 2 * (fe / EPM) * C::A_BYTES +
+                              canon_off(fe % EPM, KV + ffm, C::LBO_A);
+        if (mode == 0) {
+#pragma unroll
+          for (int c = 0; c < NU; ++c) {
+            float hi, lo;
+            split_f32((nb[c] - u0_b[c * EPB + fe]) * 0.5f, hi, lo);
+            if (reload) nb[c] = __ldg(field(c) + gn);
+            const int o = c * EPM * 16;
+            *reinterpret_cast<float*>(fdst + o) = hi;
+            *reinterpret_cast<float*>(fdst + o + C::A_BYTES) = lo;
+          }
+        } else {
+          const int64_t gm = (int64_t)(tile * EPB + fe) * NP + fk;
+          float up[NU];
+          if (mode != 2) {
+            const int bf = -((int)small_b[fe * NF + ff] + 1);
+            if (mode == 3) {
+              float nv[3] = {0.f, 0.f, 0.f}, mag2 = 0.f;
+#pragma unroll
+              for (int j = 0; j < DIM; ++j) {
+#pragma unroll
+                for (int r = 0; r < DIM; ++r)
+                  nv[j] += rx_b[fe * DD + r * DIM + j] *
+                           RefBank<float>::get(S::OFF_NREF + ff * DIM + r);
+                mag2 += nv[j] * nv[j];
+              }
+              const float mag = sqrtf(mag2);
+              mengaldo_grad_value<float, DIM, NS, true>(a, g, a.bkind[bf], bf, fm_, NFP, EN, gm,
+                                                        nv[0] / mag, nv[1] / mag, nv[2] / mag, up);
+            } else {
+              const int64_t bstride = (int64_t)a.nbf * NFP, bo = (int64_t)bf * NFP + fm_;
+#pragma unroll
+              for (int c = 0; c < NU; ++c) up[c] = a.bext[c * bstride + bo];
+            }
+          }
+#pragma unroll 1
+          for (int c = 0; c < NU; ++c) {
+            const float u0 = u0_b[c * EPB + fe];
+            const float um = __ldg(field(c) + gm) - u0;
+            float hi, lo;
+            split_f32(mode == 2 ? um * 0.5f : (up[c] - u0) - um * 0.5f, hi, lo);
+            const int o = c * EPM * 16;
+            *reinterpret_cast<float*>(fdst + o) = hi;
+            *reinterpret_cast<float*>(fdst + o + C::A_BYTES) = lo;
+          }
+        }
+      }
+      if (mode != 0 && reload) {
+#pragma unroll
+        for (int c = 0; c < NU; ++c) nb[c] = __ldg(field(c) + gn);
+      }
+      // ---- the epilogue's copy of the metric; per-tile data two tiles ahead
+      // (into the buffer of the tile before this one)
+      for (int i = tid; i < ne * DD; i += GT) geo_s[s * EPB * DD + i] = rx_b[i];
+      if (more2) small_store(w, bn == 2 ? 0 : bn + 1);
+      fence_async_shared();
+      mbar_arrive(full + s);
+      if (tid == GT - 1) pending = it;
+      b = bn;
+    }
+    // the last tile's products (after a normal end of the loop)
+    if (tid == GT - 1 && pending >= 0 && !*abort_s) issue_pending();
     // on an early exit, let the products already issued finish before the
     // TMEM is released
-    if (gtid == GT - 1 && *abort_s && issued > 0) {
+    if (tid == GT - 1 && *abort_s && issued > 0) {
       if (!mbar_wait(done + (last_issued & 1), ((uint32_t)last_issued >> 1) & 1, nullptr))
         atomicOr(a.status, ST_WAIT_TIMEOUT);
     }
@@ -638,13 +544,13 @@ __global__ void __launch_bounds__(TcGrad<DIM, ORDER, NS>::NT, 1)
     // ================= epilogue: one TMEM lane (row) per thread
     const int q4 = warp & 3;
     const int row = 32 * q4 + lane;
-    const int c = row / EPB, e = row % EPB;
+    const int c = row / EPM, el = row % EPM;
     const uint32_t lane_base = tmem + ((uint32_t)(32 * q4) << 16);
     for (int it = 0, tile = blockIdx.x; tile < ntiles; ++it, tile += gridDim.x) {
       const int s = it & 1;
       const uint32_t use = (uint32_t)it >> 1;
       // the products of this tile, then (already complete) the producers'
-      // arrival, whose release covers the geometry they wrote
+      // arrival, whose release covers the metric they wrote
       bool ok = mbar_wait(done + s, use & 1, abort_s);
       ok = ok && mbar_wait(full + s, use & 1, abort_s);
       if (!__all_sync(0xffffffffu, ok)) {
@@ -657,43 +563,41 @@ __global__ void __launch_bounds__(TcGrad<DIM, ORDER, NS>::NT, 1)
       tc_fence_after();
       const int e0 = tile * EPB;
       const int ne = imin(EPB, EOWN - e0);
-      const bool valid = c < NU && e < ne;
-      const float* ge = geo_s + s * EPB * GEO + e * GEO;
-      float rxe[DIM][DIM], nre[NF][DIM];
-#pragma unroll
-      for (int r = 0; r < DIM; ++r)
-#pragma unroll
-        for (int j = 0; j < DIM; ++j) rxe[r][j] = ge[r * DIM + j];
-#pragma unroll
-      for (int f = 0; f < NF; ++f)
-#pragma unroll
-        for (int j = 0; j < DIM; ++j) nre[f][j] = ge[DIM * DIM + f * DIM + j];
-      const uint32_t tb = lane_base + (uint32_t)(s * C::BUF_COLS);
-      float* outp = a.out + ((int64_t)(valid ? c : 0) * DIM) * EN + (int64_t)(e0 + e) * NP;
 #pragma unroll 1
-      for (int i0 = 0; i0 < NP; i0 += 4) {
-        uint32_t v[DIM + NF][4];
+      for (int mt = 0; mt < NMT; ++mt) {
+        const int e = mt * EPM + el;
+        uint32_t v[NV];
 #pragma unroll
-        for (int r = 0; r < DIM; ++r) tc_ld4(tb + r * NP + i0, v[r]);
+        for (int i = 0; i < NV; i += 16)
+          tc_ld16(lane_base + (uint32_t)(s * C::BUF_COLS + mt * NV + i), v + i);
+        tc_wait_ld<NV>(v);
+        if (c < NU && e < ne) {
+          const float* ge = geo_s + (s * EPB + e) * DD;
+          float rxe[DIM][DIM];
 #pragma unroll
-        for (int f = 0; f < NF; ++f) tc_ld4(tb + C::NV + f * NP + i0, v[DIM + f]);
-        tc_wait_ld<DIM + NF>(v);
-        if (valid) {
+          for (int r = 0; r < DIM; ++r)
 #pragma unroll
-          for (int j = 0; j < DIM; ++j) {
-            float o[4];
+            for (int j = 0; j < DIM; ++j) rxe[r][j] = ge[r * DIM + j];
+          float* outp = a.out + ((int64_t)c * DIM) * EN + (int64_t)(e0 + e) * NP;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              float gsum = 0.f;
+          for (int j = 0; j < DIM; ++j)
 #pragma unroll
-              for (int f = 0; f < NF; ++f) gsum += nre[f][j] * __uint_as_float(v[DIM + f][i]);
+            for (int i0 = 0; i0 < NP; i0 += VW) {
+              float o[VW];
 #pragma unroll
-              for (int r = 0; r < DIM; ++r) gsum -= rxe[r][j] * __uint_as_float(v[r][i]);
-              o[i] = gsum;
+              for (int i = 0; i < VW; ++i) {
+                float gsum = 0.f;
+#pragma unroll
+                for (int r = 0; r < DIM; ++r)
+                  gsum += rxe[r][j] * __uint_as_float(v[r * NP + i0 + i]);
+                o[i] = gsum;
+              }
+              float* dst = outp + (int64_t)j * EN + i0;
+              if constexpr (VW == 4)
+                *reinterpret_cast<float4*>(dst) = make_float4(o[0], o[1], o[2], o[3]);
+              else
+                *reinterpret_cast<float2*>(dst) = make_float2(o[0], o[1]);
             }
-            *reinterpret_cast<float4*>(outp + (int64_t)j * EN + i0) =
-                make_float4(o[0], o[1], o[2], o[3]);
-          }
         }
       }
       tc_fence_before();
