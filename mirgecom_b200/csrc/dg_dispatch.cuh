@@ -226,7 +226,7 @@ struct Launch {
         }
         b.grad = a.grad_out;
       }
-      const size_t smem3 = V::flux_bytes(V::EPB3, a.nperm);
+      const size_t smem3 = V::flux_bytes(V::EPB3, VISC);
       auto k3 = k_flux_volume<R, DIM, ORDER, NS, MIX, VISC>;
       rc = prepare_kernel(k3, smem3);
       if (rc) return rc;

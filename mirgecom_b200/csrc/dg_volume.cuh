@@ -42,6 +42,27 @@ namespace mgc {
 // then |v| + c, p, c, gamma, padded to 16 bytes.
 __host__ __device__ constexpr int trace_width(int nc) { return round_up(nc + 4, 4); }
 
+// The 16-byte chunks of a record are stored rotated by its slot (face slot
+// f * NFP + m; m for boundary records): the threads of a warp read the same
+// chunk of consecutive records, which would all start in the same few banks of
+// L1 (64-byte records: 4 lanes on one bank; 128-byte ones: 8).  Face kernel of
+// the reacting mixture, 32^3 p3: float32 430 -> 408 us (L1 data wavefronts 72 ->
+// 62 % of peak), float64 1129 -> 835 us (with four resident blocks instead of
+// three).
+template <class R, int TW>
+struct RecLayout {
+  static constexpr int VEC = 16 / (int)sizeof(R), NCH = TW / VEC;
+  static constexpr bool ROT = (NCH & (NCH - 1)) == 0;
+  static constexpr int PER_LINE = imax(1, 128 / (TW * (int)sizeof(R)));
+  // offset (values) of chunk t of the record in *slot*
+  static __device__ __forceinline__ int chunk(int slot, int t) {
+    return ROT ? ((t + slot / PER_LINE) & (NCH - 1)) * VEC : t * VEC;
+  }
+  static __device__ __forceinline__ int at(int slot, int i) {
+    return chunk(slot, i / VEC) + i % VEC;
+  }
+};
+
 template <class R, int DIM, int ORDER, int NS, bool MIX>
 struct VCfg {
   using G = Cfg<R, DIM, ORDER, NS, MIX>;
@@ -114,7 +135,7 @@ struct VCfg {
   // bound by its gathers' latency: 8.7 ms against 9.8 ms for four blocks of
   // 16 elements at 80^3)
   static constexpr int NT2 = 128;
-  static constexpr int MINB2 = TF32 ? 6 : 3;
+  static constexpr int MINB2 = TF32 ? 6 : 4;
   static constexpr int KFR = round_up(NFN, KSTEP);
   static constexpr int KF = Tile<R>::stride(KFR);
   static constexpr int A_FACE = NAC * MP * KF;
@@ -127,6 +148,33 @@ struct VCfg {
 };
 
 namespace {
+
+// 16-byte vector store / load of the record in *slot* (TW values, 16-byte
+// aligned)
+template <class R, int TW>
+__device__ __forceinline__ void store_rec(R* dst, int slot, const R (&rec)[TW]) {
+  using L = RecLayout<R, TW>;
+#pragma unroll
+  for (int t = 0; t < L::NCH; ++t) {
+    R* p = dst + L::chunk(slot, t);
+    if constexpr (sizeof(R) == 4)
+      *reinterpret_cast<float4*>(p) =
+          make_float4(rec[4 * t], rec[4 * t + 1], rec[4 * t + 2], rec[4 * t + 3]);
+    else
+      *reinterpret_cast<double2*>(p) = make_double2(rec[2 * t], rec[2 * t + 1]);
+  }
+}
+template <class R, int TW>
+__device__ __forceinline__ void load_rec(const R* src, int slot, R (&rec)[TW]) {
+  using L = RecLayout<R, TW>;
+#pragma unroll
+  for (int t = 0; t < L::NCH; ++t) {
+    R v[L::VEC];
+    load_record<R, L::VEC>(src + L::chunk(slot, t), v);
+#pragma unroll
+    for (int i = 0; i < L::VEC; ++i) rec[t * L::VEC + i] = v[i];
+  }
+}
 
 // The exterior state's record at face node m of prescribed boundary face bf
 // (boundary.py:141-146 for the viscous part: the exterior state with the
@@ -181,8 +229,7 @@ __device__ __noinline__ void boundary_record(const DGArgs<R> a, const GasParams 
   rec[NC + 3] = sp.gamma;
 #pragma unroll
   for (int i = NC + 4; i < TW; ++i) rec[i] = R(0);
-#pragma unroll
-  for (int i = 0; i < TW; ++i) dst[i] = rec[i];
+  store_rec<R, TW>(dst, m, rec);
 #pragma unroll
   for (int c = 0; c < NC; ++c) a.bplus[c * bstride + bo] = qp[c];
 }
@@ -256,8 +303,7 @@ __device__ __noinline__ void mengaldo_record(const DGArgs<R> a, const GasParams 
   rec[NC + 3] = sp.gamma;
 #pragma unroll
   for (int i = NC + 4; i < TW; ++i) rec[i] = R(0);
-#pragma unroll
-  for (int i = 0; i < TW; ++i) dst[i] = rec[i];
+  store_rec<R, TW>(dst, m, rec);
 #pragma unroll
   for (int c = 0; c < NC; ++c) a.bplus[c * bstride + bo] = qp[c];
 }
@@ -271,20 +317,6 @@ __device__ __forceinline__ void prefetch_l2(const void* p, size_t bytes) {
   const uintptr_t a1 = reinterpret_cast<uintptr_t>(p) + bytes;
   for (uintptr_t a = a0 + (uintptr_t)threadIdx.x * 128; a < a1; a += (uintptr_t)blockDim.x * 128)
     asm volatile("prefetch.global.L2 [%0];" ::"l"(a));
-}
-
-// 16-byte vector store / load of one record (TW values, 16-byte aligned)
-template <class R, int TW>
-__device__ __forceinline__ void store_rec(R* dst, const R (&rec)[TW]) {
-  if constexpr (sizeof(R) == 4) {
-#pragma unroll
-    for (int i = 0; i < TW; i += 4)
-      *reinterpret_cast<float4*>(dst + i) = make_float4(rec[i], rec[i + 1], rec[i + 2], rec[i + 3]);
-  } else {
-#pragma unroll
-    for (int i = 0; i < TW; i += 2)
-      *reinterpret_cast<double2*>(dst + i) = make_double2(rec[i], rec[i + 1]);
-  }
 }
 
 // Face slots f * NFP + m of each volume node (-1: none), [NP][NF], in face
@@ -649,7 +681,7 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT),
       for (int sl = 0; sl < NF; ++sl) {
         const int fm = slot_s[k * NF + sl];
         if (fm < 0) break;
-        const int f = fm / NFP, m = fm % NFP;
+        const int f = fm / NFP;
         const R* nf = nrm_s + (e * NF + f) * DIM;
         R rec[TW];
 #pragma unroll
@@ -665,7 +697,7 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT),
         rec[NC + 3] = st.gamma;
 #pragma unroll
         for (int i = NC + 4; i < TW; ++i) rec[i] = R(0);
-        store_rec<R, TW>(a.trace + (((int64_t)(e0 + e) * NF + f) * NFP + m) * TW, rec);
+        store_rec<R, TW>(a.trace + ((int64_t)(e0 + e) * NFN + fm) * TW, fm, rec);
       }
       if (k == 0) {
         // element-constant shift of the face terms: F0 . n_f, every face
@@ -896,7 +928,7 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT3), 2)
       for (int sl = 0; sl < NF; ++sl) {
         const int fm = slot_s[k * NF + sl];
         if (fm < 0) break;
-        const int f = fm / NFP, m = fm % NFP;
+        const int f = fm / NFP;
         const R* nf = nrm_s + (e * NF + f) * DIM;
         R rec[TW];
 #pragma unroll
@@ -912,7 +944,7 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT3), 2)
         rec[NC + 3] = st.gamma;
 #pragma unroll
         for (int i = NC + 4; i < TW; ++i) rec[i] = R(0);
-        store_rec<R, TW>(a.trace + (((int64_t)(e0 + e) * NF + f) * NFP + m) * TW, rec);
+        store_rec<R, TW>(a.trace + ((int64_t)(e0 + e) * NFN + fm) * TW, fm, rec);
       }
       if (k == 0) {
         R* s0e = a.s0 + (int64_t)(e0 + e) * NF * NC;
@@ -1101,20 +1133,23 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT3), 2)
 // neighbour-convention records; qp_g: the exterior q (stride qstride).
 template <class R, int DIM, int NS, bool VISC>
 __device__ __noinline__ void face_flux_general(const DGArgs<R> a, int64_t EN, int64_t gm,
-                                               const R* recm, const R* recp, const R* qp_g,
+                                               const R* recm, int slm, const R* recp, int slp,
+                                               const R* qp_g,
                                                int64_t qstride, R n0, R n1, R n2, R fsc,
                                                const R* s0, R* bcol, int cstride) {
-  constexpr int NC = DIM + 2 + NS;
+  constexpr int NC = DIM + 2 + NS, TW = trace_width(NC);
   const R n[3] = {n0, n1, n2};
-  R qm[NC], qp[NC];
+  R qm[NC], qp[NC], rm[TW], rp[TW];
+  load_rec<R, TW>(recm, slm, rm);
+  load_rec<R, TW>(recp, slp, rp);
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
     qm[c] = a.q[c * EN + gm];
     qp[c] = qp_g[c * qstride];
   }
   NodeState<R, DIM, NS> sm, sp;
-  make_state_light<R, DIM, NS>(qm, recm[NC + 1], recm[NC + 2], recm[NC + 3], sm);
-  make_state_light<R, DIM, NS>(qp, recp[NC + 1], recp[NC + 2], recp[NC + 3], sp);
+  make_state_light<R, DIM, NS>(qm, rm[NC + 1], rm[NC + 2], rm[NC + 3], sm);
+  make_state_light<R, DIM, NS>(qp, rp[NC + 1], rp[NC + 2], rp[NC + 3], sp);
   R fi[NC], fim[NC], fip[NC];
   inviscid_num_flux<R, DIM, NS>(sm, sp, qm, qp, n, FLUX_HLL, fi);
   inviscid_flux_n<R, DIM, NS>(sm, n, fim);
@@ -1123,9 +1158,9 @@ __device__ __noinline__ void face_flux_general(const DGArgs<R> a, int64_t EN, in
   for (int c = 0; c < NC; ++c) {
     R out = -fi[c];
     // F_V . n = F . n + F_I . n on each side; the neighbour record holds -F . n
-    if (VISC) out += ((recm[c] + fim[c]) + (-recp[c] + fip[c])) * R(0.5);
+    if (VISC) out += ((rm[c] + fim[c]) + (-rp[c] + fip[c])) * R(0.5);
     // less the shift and the own half that WH carries
-    bcol[c * cstride] = fsc * (folds<R>() ? out - (recm[c] + s0[c]) * R(0.5) : out - s0[c]);
+    bcol[c * cstride] = fsc * (folds<R>() ? out - (rm[c] + s0[c]) * R(0.5) : out - s0[c]);
   }
 }
 
@@ -1186,13 +1221,13 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT2),
       const int cn = conn_s[e * NF + f];
       const R fsc = fs_s[e * NF + f];
       const int64_t gm = (int64_t)(e0 + e) * NP + k;
-      const R* recm = a.trace + (((int64_t)(e0 + e) * NF + f) * NFP + m) * TW;
+      const R* recm = a.trace + ((int64_t)(e0 + e) * NFN + fm) * TW;
       const R* s0 = a.s0 + ((int64_t)(e0 + e) * NF + f) * NC;
       R* bcol = bm + e * KF + fm;
       // neighbour record and exterior q; mode 0 interior, 1 prescribed,
       // 2 interior flux only (dummy boundary, or a pairing that fails its
       // index checks)
-      int mode = 2;
+      int mode = 2, slp = 0;
       const R* recp = nullptr;
       const R* qp_g = nullptr;
       int64_t qstride = EN;
@@ -1205,6 +1240,7 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT2),
         }
         if (en < E && kn < NP && sl < NFN) {
           recp = a.trace + ((int64_t)en * NFN + sl) * TW;
+          slp = sl;
           qp_g = a.q + (int64_t)en * NP + kn;
           mode = 0;
         } else {
@@ -1217,6 +1253,7 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT2),
         if (kind >= BK_PRESCRIBED) {
           // the volume kernel filed the exterior record and state_plus
           recp = a.btrace + ((int64_t)bf * NFP + m) * TW;
+          slp = m;
           qp_g = a.bplus + (int64_t)bf * NFP + m;
           qstride = bstride;
           mode = 1;
@@ -1226,28 +1263,42 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT2),
       }
       if (mode == 2) {
         // DummyBoundary: F* = F(q-) . n (boundary.py:1027-1049)
+        R rm[TW];
+        load_rec<R, TW>(recm, fm, rm);
 #pragma unroll
         for (int c = 0; c < NC; ++c)
-          bcol[c * EPB * KF] = (folds<R>() ? fsc * R(0.5) : fsc) * (recm[c] - s0[c]);
+          bcol[c * EPB * KF] = (folds<R>() ? fsc * R(0.5) : fsc) * (rm[c] - s0[c]);
         continue;
       }
       if (a.flux_kind == FLUX_HLL) {
         const R* nf = nrm_s + (e * NF + f) * DIM;
-        face_flux_general<R, DIM, NS, VISC>(a, EN, gm, recm, recp, qp_g, qstride, nf[0], nf[1],
+        face_flux_general<R, DIM, NS, VISC>(a, EN, gm, recm, fm, recp, slp, qp_g, qstride, nf[0], nf[1],
                                             DIM > 2 ? nf[DIM - 1] : R(0), fsc, s0, bcol,
                                             EPB * KF);
         continue;
       }
       R rm[TW], rp[TW];
-      if constexpr (!folds<R>()) load_record<R, TW>(recm, rm);
-      load_record<R, TW>(recp, rp);
+      if constexpr (!folds<R>()) load_rec<R, TW>(recm, fm, rm);
+      load_rec<R, TW>(recp, slp, rp);
       const R lamm = folds<R>() ? a.lam[gm] : rm[NC];
       R qm[NC], qp[NC], sh[NC];
+      constexpr int VEC = RecLayout<R, TW>::VEC;
+      if constexpr (NC % VEC == 0) {
+#pragma unroll
+        for (int c = 0; c < NC; c += VEC) {
+          R v[VEC];
+          load_record<R, VEC>(s0 + c, v);
+#pragma unroll
+          for (int i = 0; i < VEC; ++i) sh[c + i] = v[i];
+        }
+      } else {
+#pragma unroll
+        for (int c = 0; c < NC; ++c) sh[c] = s0[c];
+      }
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
         qm[c] = a.q[c * EN + gm];
         qp[c] = qp_g[c * qstride];
-        sh[c] = s0[c];
       }
       const R lam = (a.flux_kind == FLUX_RUSANOV) ? fmax(lamm, rp[NC]) : R(0);
       if constexpr (folds<R>()) {
