@@ -33,6 +33,7 @@
 // leaves the discrete divergence unchanged: -W c + LIFT (c.n) = 0 for a
 // constant c, so -WH c + LIFT (c.n) / 2 = 0.
 #pragma once
+#include "async_copy.cuh"
 #include "boundary.cuh"
 #include "dg_kernels.cuh"
 
@@ -112,19 +113,31 @@ struct VCfg {
   static constexpr int NCOLD = round_up(NC * EPB, 8);      // divergence columns
 
   // ---- flux-volume kernel (gradients from HBM): no gradient operands or
-  // staging; element tiles sized so the pointwise phase fills the block
+  // staging of its own gradients; element tiles sized so the pointwise phase
+  // fills the block.  The tile's inputs are staged in shared memory: rows of
+  // the NC fields, the operator and source temperatures, the gradients
   static constexpr int NT3 = TF32 ? 256 : 128;
-  static constexpr int A_FLUX = NAC * DIM * MP * KU;
-  static constexpr __host__ __device__ int nnode3(int epb) { return epb * NP + (KUR - NP) + 4; }
-  static constexpr __host__ __device__ size_t flux_bytes(int epb, int nperm) {
-    return (size_t)(A_FLUX + nnode3(epb) * FST + NS * epb * NP + epb * GEO) * RB + NFN * 4 +
-           epb * NF * 4 + NP * NF * 2 + (size_t)nperm * NFP + 64;
+  // operator rows: NP per r.  The last m-tile reads up to MP rows, on into the
+  // next matrix or gfl (accumulator rows >= NP, never stored)
+  static constexpr int A_FLUX = NAC * DIM * NP * KU;
+  static constexpr int ROW_T = NC, ROW_G = NC + (MIX ? 2 : 0);
+  static constexpr __host__ __device__ int rows3(bool visc) {
+    return ROW_G + (visc ? NU * DIM : 0);
   }
-  // the largest tile with at most one node per thread and two blocks per SM
+  static constexpr int GEO3 = DIM * DIM + NF * DIM;        // metric, unit normals
+  static constexpr __host__ __device__ int nnode3(int epb) { return epb * NP + (KUR - NP) + 4; }
+  static constexpr __host__ __device__ size_t flux_bytes(int epb, bool visc) {
+    return (size_t)round_up(A_FLUX + nnode3(epb) * FST + NS * epb * NP + 2 * epb * GEO3 +
+                                epb * NC * DIM, 4) * RB +
+           (size_t)round_up(epb * NP * RB, 16) * rows3(visc) + NFN * 4 + 2 * epb * NF * 4 +
+           NP * NF * 2 + 64;
+  }
+  // the largest tile with at most one node per thread and two blocks per SM;
+  // even, so that rows of NP even values start on 16 bytes
   static constexpr __host__ __device__ int pick_epb3() {
     int best = 1;
-    for (int e = 1; e * NP <= NT3; ++e)
-      if (flux_bytes(e, 32) <= (size_t)BUDGET) best = e;
+    for (int e = 2; e * NP <= NT3; e += 2)
+      if (flux_bytes(e, true) <= (size_t)BUDGET) best = e;
     return best;
   }
   static constexpr int EPB3 = pick_epb3();
@@ -821,10 +834,21 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT),
 }
 
 // Flux-volume kernel: the pointwise phase and the volume divergence of
-// k_volume with the gradients read from HBM (written by k_grad), for the
-// three-kernel pass gradient -> flux-volume -> face.  Without the gradient
-// operands and staging its tiles fill the block: 12 order-3 tetrahedra (240
-// nodes) per 256 threads on the float32 path.
+// k_volume with the gradients read from HBM (written by the gradient kernel),
+// for the three-kernel pass gradient -> flux-volume -> face.
+//
+// The tile's inputs (NC fields, temperatures, (NC+1) DIM gradients: one
+// contiguous row of EPB * NP values each) are brought into shared memory by
+// bulk copies (cp.async.bulk), issued as soon as the previous tile's pointwise
+// phase has read its own and running under that tile's divergence; its
+// geometry is computed in the same window into a second buffer.  A node's
+// thread then reads them where the flux needs them: no address arithmetic, no
+// registers held for loads in flight, no wait for DRAM at the start of a tile.
+// Rows that bulk copies cannot move (a row start off 16 bytes: odd NP, an odd
+// number of order-2 float32 elements, an unaligned caller's pointer) are
+// copied by the threads into the same place.  Measured: float64 32^3 p3 2.57 ->
+// 2.46 ms, float32 1260 tetrahedra 23.5 -> 20.2 us; float32 64^3 p3 is the same
+// with and without (7.46 ms: its pointwise arithmetic bounds it).
 template <class R, int DIM, int ORDER, int NS, bool MIX, bool VISC>
 __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT3), 2)
     k_flux_volume(DGArgs<R> a, GasParams g) {
@@ -833,52 +857,137 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT3), 2)
   constexpr int NP = V::NP, NF = V::NF, NFP = V::NFP, NFN = V::NFN, NC = V::NC;
   constexpr int EPB = V::EPB3, MP = V::MP, MT = V::MT, MROW = V::MROW;
   constexpr int KU = V::KU, KUR = V::KUR, NCOLD = V::NCOL3, NNODE = V::nnode3(V::EPB3);
-  constexpr int FST = V::FST, TW = V::TW;
-  constexpr int AWN = DIM * MP * KU;
+  constexpr int FST = V::FST, TW = V::TW, GEO = V::GEO3, DD = DIM * DIM;
+  constexpr int AWN = DIM * NP * KU;
   constexpr int ENP = EPB * NP;
+  constexpr int NROW = V::rows3(VISC), RST = round_up(ENP * (int)sizeof(R), 16) / (int)sizeof(R);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   R* aw = reinterpret_cast<R*>(smem_raw);                  // [NAC][DIM][MP][KU]
   R* gfl = aw + V::A_FLUX;                                 // [NNODE][FST]
   R* src_s = gfl + NNODE * FST;                            // [NS][ENP]
-  R* rx_s = src_s + NS * ENP;                              // [EPB][DIM][DIM]
-  R* nrm_s = rx_s + EPB * DIM * DIM;                       // [EPB][NF][DIM]
-  R* fs_s = nrm_s + EPB * NF * DIM;                        // [EPB][NF]
-  int* fn_s = reinterpret_cast<int*>(fs_s + EPB * NF);     // [NFN]
-  int32_t* conn_s = fn_s + NFN;                            // [EPB][NF]
-  int16_t* slot_s = reinterpret_cast<int16_t*>(conn_s + EPB * NF);   // [NP][NF]
+  R* geo_s = src_s + NS * ENP;                             // [2][EPB][GEO]
+  R* f0_s = geo_s + 2 * EPB * GEO;                         // [EPB][NC * DIM] node-0 fluxes
+  R* row_s = aw + round_up(V::A_FLUX + NNODE * FST + NS * ENP + 2 * EPB * GEO + EPB * NC * DIM,
+                           4);                             // [NROW][RST]
+  int* fn_s = reinterpret_cast<int*>(row_s + NROW * RST);  // [NFN]
+  int32_t* conn_s = fn_s + NFN;                            // [2][EPB][NF]
+  int16_t* slot_s = reinterpret_cast<int16_t*>(conn_s + 2 * EPB * NF);   // [NP][NF]
+  __shared__ __align__(8) uint64_t staged;                 // the tile's rows have landed
 
-  const int E = a.nelem;
-  const int64_t EN = (int64_t)E * NP;
+  const int64_t EN = (int64_t)a.nelem * NP;
   const bool sources = MIX && a.add_sources;
+  // float32 drivers pass one temperature for both uses
+  const bool own_src = sources && a.t_src != a.t_op;
+  auto row_ptr = [&](int i) -> const R* {
+    if (i < NC) return a.q + i * EN;
+    if (MIX && i < V::ROW_G) return i == V::ROW_T ? a.t_op : (own_src ? a.t_src : nullptr);
+    return a.grad + (i - V::ROW_G) * EN;
+  };
+  const bool bulk = ((reinterpret_cast<uintptr_t>(a.q) | (MIX ? reinterpret_cast<uintptr_t>(a.t_op) : 0) |
+                      (own_src ? reinterpret_cast<uintptr_t>(a.t_src) : 0) |
+                      (VISC ? reinterpret_cast<uintptr_t>(a.grad) : 0)) & 15) == 0 &&
+                    (EN * sizeof(R)) % 16 == 0 && (ENP * sizeof(R)) % 16 == 0;
+  const int ntiles = (a.nowned + EPB - 1) / EPB;
+  // rows of tile *tl*: bulk copies by warp 0 (all threads without them)
+  auto stage_rows = [&](int tl) {
+    const int64_t n0 = (int64_t)tl * ENP;
+    const int n = imin(ENP, (int)((int64_t)a.nowned * NP - n0));
+    int done_n = 0;
+    if (bulk) {
+      const uint32_t bytes = (uint32_t)(n * sizeof(R)) & ~15u;
+      done_n = bytes / (int)sizeof(R);
+      if (threadIdx.x < 32) {
+        if (threadIdx.x == 0)
+          mbar_expect(&staged, bytes * (uint32_t)(NROW - (MIX && !own_src ? 1 : 0)));
+        __syncwarp();
+        for (int i = threadIdx.x; i < NROW; i += 32) {
+          const R* p = row_ptr(i);
+          if (p && bytes) bulk_load(row_s + i * RST, p + n0, bytes, &staged);
+        }
+      }
+    }
+    if (done_n < n) {
+      const int m = n - done_n;
+      for (int i = threadIdx.x; i < NROW * m; i += blockDim.x) {
+        const R* p = row_ptr(i / m);
+        if (p) row_s[(i / m) * RST + done_n + i % m] = p[n0 + done_n + i % m];
+      }
+    }
+  };
+  // geometry and face pairing of tile *tl* into buffer *b*, by the threads
+  // [t0, t0 + nt): metric and unit normals as load_geometry computes them
+  auto geometry = [&](int tl, int b, int t0, int nt) {
+    const int e1 = tl * EPB, n1 = imin(EPB, a.nowned - e1);
+    R* gb = geo_s + b * EPB * GEO;
+    for (int i = (int)threadIdx.x - t0; i < n1 * NF; i += nt) {
+      if (i < 0) break;
+      const int e = i / NF, f = i % NF;
+      conn_s[b * EPB * NF + i] = a.conn[(int64_t)e1 * NF + i];
+      const R* rxg = a.rx + (int64_t)(e1 + e) * DD;
+      R rx[DD];
+#pragma unroll
+      for (int k = 0; k < DD; ++k) rx[k] = rxg[k];
+      R nv[DIM], mag2 = 0;
+#pragma unroll
+      for (int j = 0; j < DIM; ++j) {
+        R s = 0;
+#pragma unroll
+        for (int r = 0; r < DIM; ++r)
+          s += rx[r * DIM + j] * RefBank<R>::get(S::OFF_NREF + f * DIM + r);
+        nv[j] = s;
+        mag2 += s * s;
+      }
+      const R mag = sqrt(mag2);
+#pragma unroll
+      for (int j = 0; j < DIM; ++j) gb[e * GEO + DD + f * DIM + j] = nv[j] / mag;
+      if (f == 0) {
+#pragma unroll
+        for (int k = 0; k < DD; ++k) gb[e * GEO + k] = rx[k];
+      }
+    }
+  };
+
+  if (threadIdx.x == 0) {
+    mbar_init(&staged, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
   for (int i = threadIdx.x; i < AWN; i += blockDim.x) {
-    const int r = i / (MP * KU), row = (i / KU) % MP, k = i % KU;
-    put_a<R>(aw, AWN, i, (row < NP && k < NP) ? refop(S::template OFF_WDIV<R> + (r * NP + row) * NP + k) : 0.0);
+    const int k = i % KU, row = i / KU;                    // row = r * NP + output node
+    put_a<R>(aw, AWN, i, k < NP ? refop(S::template OFF_WDIV<R> + row * NP + k) : 0.0);
   }
   for (int i = threadIdx.x; i < NNODE * FST + NS * ENP; i += blockDim.x) gfl[i] = R(0);
   for (int i = threadIdx.x; i < NFN; i += blockDim.x) fn_s[i] = c_face_nodes<DIM, ORDER>(i);
   fill_slots<DIM, ORDER>(slot_s);
+  __syncthreads();
+  if ((int)blockIdx.x < ntiles) {
+    stage_rows(blockIdx.x);
+    geometry(blockIdx.x, 0, 0, blockDim.x);
+  }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gq = lane >> 2, tq = lane & 3;
   const int nwarps = blockDim.x >> 5;
   constexpr int NACC = V::TF32 ? 4 : 2;
-  const int ntiles = (a.nowned + EPB - 1) / EPB;
   bool bad = false;
-  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+  int it = 0;
+  bool timeout = false;
+  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++it) {
+    const int b = it & 1;
     const int e0 = tile * EPB;
     const int ne = imin(EPB, a.nowned - e0);
+    const R* gb = geo_s + b * EPB * GEO;
+    // the previous tile's divergence has read gfl and src_s; this tile's
+    // geometry is complete
     __syncthreads();
-    stage_conn<NF>(a.conn, e0, ne, conn_s);
-    load_geometry<R, DIM, ORDER>(a.rx, e0, ne, rx_s, nrm_s, fs_s);
-    __syncthreads();
+    const bool ok = !bulk || mbar_wait(&staged, it & 1, nullptr);
 
-    for (int n = threadIdx.x; n < ne * NP; n += blockDim.x) {
+    for (int n = threadIdx.x; n < ne * NP && ok; n += blockDim.x) {
       const int e = n / NP, k = n % NP;
       const int64_t gnd = (int64_t)(e0 + e) * NP + k;
       R qq[NC];
 #pragma unroll
-      for (int c = 0; c < NC; ++c) qq[c] = a.q[c * EN + gnd];
+      for (int c = 0; c < NC; ++c) qq[c] = row_s[c * RST + n];
       NodeState<R, DIM, NS> st;
-      make_state<R, DIM, NS>(qq, MIX ? a.t_op[gnd] : R(0), g, st);
+      make_state<R, DIM, NS>(qq, MIX ? row_s[V::ROW_T * RST + n] : R(0), g, st);
       R fl[NC][DIM];
       inviscid_flux<R, DIM, NS>(st, fl);
 #pragma unroll
@@ -886,13 +995,14 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT3), 2)
 #pragma unroll
         for (int j = 0; j < DIM; ++j) fl[c][j] = -fl[c][j];
       if constexpr (VISC) {
+        const R* gr = row_s + V::ROW_G * RST + n;
         R gqv[NC][DIM], gt[DIM];
 #pragma unroll
         for (int c = 0; c < NC; ++c)
 #pragma unroll
-          for (int j = 0; j < DIM; ++j) gqv[c][j] = a.grad[((int64_t)c * DIM + j) * EN + gnd];
+          for (int j = 0; j < DIM; ++j) gqv[c][j] = gr[(c * DIM + j) * RST];
 #pragma unroll
-        for (int j = 0; j < DIM; ++j) gt[j] = a.grad[((int64_t)NC * DIM + j) * EN + gnd];
+        for (int j = 0; j < DIM; ++j) gt[j] = gr[(NC * DIM + j) * RST];
         R fv[NC][DIM];
         viscous_flux<R, DIM, NS, MIX>(st, gqv, gt, fv);
 #pragma unroll
@@ -901,7 +1011,7 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT3), 2)
           for (int j = 0; j < DIM; ++j) fl[c][j] = fv[c][j] + fl[c][j];
       }
       bad |= !(st.p == st.p) || !(st.c == st.c);
-      const R* rxe = rx_s + e * DIM * DIM;
+      const R* rxe = gb + e * GEO;
 #pragma unroll
       for (int c = 0; c < NC; ++c)
 #pragma unroll
@@ -914,7 +1024,8 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT3), 2)
       if constexpr (MIX && NS > 0) {
         if (sources) {
           R om[NS];
-          production_rates<R, NS>(st.rho, a.t_src[gnd], st.y, (R)g.zero_level, om);
+          production_rates<R, NS>(st.rho, row_s[(own_src ? V::ROW_T + 1 : V::ROW_T) * RST + n],
+                                  st.y, (R)g.zero_level, om);
 #pragma unroll
           for (int sp = 0; sp < NS; ++sp) src_s[sp * ENP + n] = mech<R>().mw[sp] * om[sp];
         }
@@ -928,8 +1039,7 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT3), 2)
       for (int sl = 0; sl < NF; ++sl) {
         const int fm = slot_s[k * NF + sl];
         if (fm < 0) break;
-        const int f = fm / NFP;
-        const R* nf = nrm_s + (e * NF + f) * DIM;
+        const R* nf = gb + e * GEO + DD + (fm / NFP) * DIM;
         R rec[TW];
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
@@ -947,42 +1057,57 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT3), 2)
         store_rec<R, TW>(a.trace + ((int64_t)(e0 + e) * NFN + fm) * TW, fm, rec);
       }
       if (k == 0) {
-        R* s0e = a.s0 + (int64_t)(e0 + e) * NF * NC;
-#pragma unroll 1
-        for (int f = 0; f < NF; ++f) {
-          const R* nf = nrm_s + (e * NF + f) * DIM;
 #pragma unroll
-          for (int c = 0; c < NC; ++c) {
-            R acc = R(0);
+        for (int c = 0; c < NC; ++c)
 #pragma unroll
-            for (int j = 0; j < DIM; ++j) acc += fl[c][j] * nf[j];
-            s0e[f * NC + c] = acc;
-          }
-        }
+          for (int j = 0; j < DIM; ++j) f0_s[e * NC * DIM + c * DIM + j] = fl[c][j];
       }
     }
     // exterior records of the tile's boundary face nodes (own loop: see k_volume)
-    for (int fnode = threadIdx.x; fnode < ne * NFN; fnode += blockDim.x) {
-      const int e = fnode / NFN, fm = fnode % NFN, f = fm / NFP, m = fm % NFP;
-      const int cn = conn_s[e * NF + f];
-      if (cn >= 0) continue;
-      const int bf = -(cn + 1);
-      const int kind = (bf < a.nbf) ? a.bkind[bf] : -1;
-      if ((bk_needs_bext(kind) && !a.bext) || (kind != BK_PRESCRIBED && !bk_mengaldo(kind)))
-        continue;
-      const int64_t gnd = (int64_t)(e0 + e) * NP + fn_s[fm];
-      const R* nf = nrm_s + (e * NF + f) * DIM;
-      R* dst = a.btrace + ((int64_t)bf * NFP + m) * TW;
-      if (kind == BK_PRESCRIBED)
-        boundary_record<R, DIM, NS, MIX, VISC>(a, g, bf, m, NFP, VISC ? a.grad + gnd : nullptr,
-                                               EN, nf[0], nf[1], DIM > 2 ? nf[DIM - 1] : R(0),
-                                               dst);
-      else
-        mengaldo_record<R, DIM, NS, MIX, VISC>(a, g, kind, bf, m, NFP, EN, gnd,
-                                               VISC ? a.grad + gnd : nullptr, EN, nf[0], nf[1],
-                                               DIM > 2 ? nf[DIM - 1] : R(0), dst);
+    if (a.nbf > 0) {
+      for (int fnode = threadIdx.x; fnode < ne * NFN && ok; fnode += blockDim.x) {
+        const int e = fnode / NFN, fm = fnode % NFN, f = fm / NFP, m = fm % NFP;
+        const int cn = conn_s[(b * EPB + e) * NF + f];
+        if (cn >= 0) continue;
+        const int bf = -(cn + 1);
+        const int kind = (bf < a.nbf) ? a.bkind[bf] : -1;
+        if ((bk_needs_bext(kind) && !a.bext) || (kind != BK_PRESCRIBED && !bk_mengaldo(kind)))
+          continue;
+        const int64_t gnd = (int64_t)(e0 + e) * NP + fn_s[fm];
+        const R* nf = gb + e * GEO + DD + f * DIM;
+        R* dst = a.btrace + ((int64_t)bf * NFP + m) * TW;
+        if (kind == BK_PRESCRIBED)
+          boundary_record<R, DIM, NS, MIX, VISC>(a, g, bf, m, NFP, VISC ? a.grad + gnd : nullptr,
+                                                 EN, nf[0], nf[1], DIM > 2 ? nf[DIM - 1] : R(0),
+                                                 dst);
+        else
+          mengaldo_record<R, DIM, NS, MIX, VISC>(a, g, kind, bf, m, NFP, EN, gnd,
+                                                 VISC ? a.grad + gnd : nullptr, EN, nf[0], nf[1],
+                                                 DIM > 2 ? nf[DIM - 1] : R(0), dst);
+      }
     }
-    __syncthreads();
+    // gfl and the sources are complete, the staged rows have been read
+    if (__syncthreads_or(!ok)) {
+      timeout = true;
+      break;
+    }
+    if (tile + (int)gridDim.x < ntiles) {
+      stage_rows(tile + gridDim.x);
+      // by the last warps, which have the least divergence work
+      geometry(tile + gridDim.x, b ^ 1, blockDim.x - 64, 64);
+    }
+    // element-constant shift of the face terms, F0 . n of every face, by the
+    // same warps (by the node-0 threads it took each warp ~350 instructions
+    // for one or two lanes)
+    for (int i = (int)threadIdx.x - (int)blockDim.x + 64; i >= 0 && i < ne * NF * NC; i += 64) {
+      const int c = i % NC, f = (i / NC) % NF, e = i / (NC * NF);
+      const R* f0 = f0_s + (e * NC + c) * DIM;
+      const R* nf = gb + e * GEO + DD + f * DIM;
+      R acc = R(0);
+#pragma unroll
+      for (int j = 0; j < DIM; ++j) acc += f0[j] * nf[j];
+      a.s0[(int64_t)e0 * NF * NC + i] = acc;
+    }
 
     // volume divergence.  float32: one item per group of NTG column tiles
     // and every m-tile, so each shifted flux value is read and split into
@@ -1027,8 +1152,8 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT3), 2)
 #pragma unroll
             for (int t = 0; t < MT; ++t) {
               uint32_t ah[4], alo[4];
-              load_a_tf32_ldsm(ah, aw + r * MP * KU, KU, t * 16, ks * 8, lane);
-              load_a_tf32_ldsm(alo, aw + AWN + r * MP * KU, KU, t * 16, ks * 8, lane);
+              load_a_tf32_ldsm(ah, aw + r * NP * KU, KU, t * 16, ks * 8, lane);
+              load_a_tf32_ldsm(alo, aw + AWN + r * NP * KU, KU, t * 16, ks * 8, lane);
 #pragma unroll
               for (int u = 0; u < NTG; ++u) mma_tf32x3(d[t][u], ah, alo, bs[u]);
             }
@@ -1077,7 +1202,7 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT3), 2)
         if constexpr (!V::TF32) {
 #pragma unroll
           for (int ks = 0; ks < KUR / 4; ++ks) {
-            const double av = aw[(r * MP + t * 8 + gq) * KU + ks * 4 + tq];
+            const double av = aw[(r * NP + t * 8 + gq) * KU + ks * 4 + tq];
             const int kk = ks * 4 + tq;
 #pragma unroll
             for (int u = 0; u < NTG; ++u) {
@@ -1089,8 +1214,8 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT3), 2)
 #pragma unroll
           for (int ks = 0; ks < KUR / 8; ++ks) {
             uint32_t ah[4], alo[4];
-            load_a_tf32_ldsm(ah, aw + r * MP * KU, KU, t * 16, ks * 8, lane);
-            load_a_tf32_ldsm(alo, aw + AWN + r * MP * KU, KU, t * 16, ks * 8, lane);
+            load_a_tf32_ldsm(ah, aw + r * NP * KU, KU, t * 16, ks * 8, lane);
+            load_a_tf32_ldsm(alo, aw + AWN + r * NP * KU, KU, t * 16, ks * 8, lane);
             const int k0 = ks * 8 + tq;
 #pragma unroll
             for (int u = 0; u < NTG; ++u) {
@@ -1122,6 +1247,11 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT3), 2)
           }
         }
     }
+  }
+  if (timeout && threadIdx.x == 0) {
+    atomicOr(a.status, ST_WAIT_TIMEOUT);
+    // the copies in flight end before the block does
+    if (!mbar_wait(&staged, it & 1, nullptr)) atomicOr(a.status, ST_WAIT_TIMEOUT);
   }
   if (bad) atomicOr(a.status, ST_NAN);
 }
