@@ -39,6 +39,9 @@ inline Mechanism expand_mechanism(const mgc_mechanism_t& m) {
       e[5] = a[6];
     }
   }
+  d.one_t_mid = 1;
+  for (int s = 1; s < m.nspecies && s < MGC_MAX_SPECIES; ++s)
+    if (m.t_mid[s] != m.t_mid[0]) d.one_t_mid = 0;
   // Newton convergence constant: max over species and T in [200, 6000] K of
   // |c_v'| / (2 c_v), c_v/R = a0 - 1 + a1 T + ... + a4 T^4 (1 K steps)
   double kmax = 0.0;

@@ -427,16 +427,18 @@ __global__ void __launch_bounds__(256) k_mixture_state_mixed(
     float qq[NC];
 #pragma unroll
     for (int c = 0; c < NC; ++c) qq[c] = q[(int64_t)c * nnodes + n];
-    float y[NS], e32;
-    double yd[NS], e64;
-    mixed_newton_inputs<DIM, NS>(qq, y, yd, e32, e64);
+    MixedEnergy<NS> en;
+    double e64;
+    mixed_newton_inputs<DIM, NS>(qq, en.yw, e64);
+    const float e32 = (float)e64;
+    en.start(tguess ? tguess[n] : tseed[n]);
     int used = 0;
     float t = 0.f;
     bool ok = false;
     // attempt 0: learned guess (when given); attempt 1: the plain guess (seed)
     for (int attempt = tguess ? 0 : 1; attempt < 2 && !ok; ++attempt) {
       t = (attempt == 0) ? tguess[n] : tseed[n];
-      ok = mixed_newton<NS>(y, yd, e32, e64, t, maxit, (double)rtol, used);
+      ok = mixed_newton<NS>(en, e32, e64, t, maxit, (double)rtol, used);
       if (!ok && attempt == 0) used += 1000;
     }
     if (!ok) miss = true;

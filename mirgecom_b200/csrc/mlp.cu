@@ -594,13 +594,15 @@ __global__ void __launch_bounds__(WARPS * 32, 6) k_mixture_state_learned(
     float qq[NC];
 #pragma unroll
     for (int c = 0; c < NC; ++c) qq[c] = valid ? q[(int64_t)c * n + s] : (c == 0 ? 1.f : 0.f);
-    float y[NS], e32;
-    double yd[NS], e64;
-    mixed_newton_inputs<DIM, NS>(qq, y, yd, e32, e64);
+    MixedEnergy<NS> en;
+    double e64;
+    mixed_newton_inputs<DIM, NS>(qq, en.yw, e64);
+    const float e32 = (float)e64;
     // one float32 step from the seed; a warm warp continues from there
     const float ts = valid ? tseed[s] : 1000.f;
     float t, em, cv;
-    mixture_e_cv<float, NS>(y, ts, em, cv);
+    en.start(ts);
+    en.eval(ts, em, cv);
     const float dt0 = (e32 - em) / cv;
     int used, mx;
     if (__all_sync(0xffffffffu, !valid || (ts > 0.f && fabsf(dt0) <= kWarmSeedK))) {
@@ -613,7 +615,7 @@ __global__ void __launch_bounds__(WARPS * 32, 6) k_mixture_state_learned(
       float f[8];
       f[0] = e32;
 #pragma unroll
-      for (int k = 0; k < 7; ++k) f[1 + k] = k < NS ? y[k] : 0.f;
+      for (int k = 0; k < 7; ++k) f[1 + k] = k < NS ? (float)(en.yw[k] * mech<double>().mw[k]) : 0.f;
 #pragma unroll
       for (int j = 0; j < KIN; j += 2) {
         const float v0 = j < 8 ? (f[j] - net.in_shift[j]) * net.in_scale[j] : 0.f;
@@ -640,14 +642,15 @@ __global__ void __launch_bounds__(WARPS * 32, 6) k_mixture_state_learned(
       // so that none of them stays live across the network
 #pragma unroll
       for (int c = 0; c < NC; ++c) qq[c] = valid ? q[(int64_t)c * n + s] : (c == 0 ? 1.f : 0.f);
-      mixed_newton_inputs<DIM, NS>(qq, y, yd, e32, e64);
+      mixed_newton_inputs<DIM, NS>(qq, en.yw, e64);
+      en.start(t);
     }
     if (valid) {
-      bool ok = mixed_newton<NS>(y, yd, e32, e64, t, mx, rtol, used);
+      bool ok = mixed_newton<NS>(en, e32, e64, t, mx, rtol, used);
       if (!ok) {
         used += 1000;
         t = ts;
-        ok = mixed_newton<NS>(y, yd, e32, e64, t, maxit, rtol, used);
+        ok = mixed_newton<NS>(en, e32, e64, t, maxit, rtol, used);
       }
       if (!ok) miss = true;
       tout[s] = t;
