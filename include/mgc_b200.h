@@ -246,6 +246,15 @@ int mgc_rhs_split_f32(int viscous, const mgc_mesh_t* mesh, const mgc_gas_t* gas,
                       void* workspace, size_t workspace_bytes, int32_t* status, void* stream,
                       void* mid_event);
 
+/* euler_operator (viscous = 0) or ns_operator (viscous = 1) on tensor-product
+ * hexahedra, ideal gas, float64, without storing the gradients: a volume
+ * kernel and a face kernel (mid_event recorded between them).  The workspace
+ * is mgc_rhs_split_workspace_bytes(mesh, gas, 0) bytes, 256-byte aligned;
+ * mesh->fslot is required.  Same results as mgc_ns_grad + mgc_rhs_split. */
+int mgc_rhs_hex(int viscous, const mgc_mesh_t* mesh, const mgc_gas_t* gas, const double* q,
+                const double* bext, int flux_kind, double* rhs, void* workspace,
+                size_t workspace_bytes, int32_t* status, void* stream, void* mid_event);
+
 /* Gradient-pass kernel of every entry point that computes gradients
  * (mgc_ns_grad*, mgc_ns_rhs*'s callers, mgc_operator* with phases bit 4):
  * MGC_GRAD_AUTO (default) runs the tcgen05/TMEM pipelined kernel where it

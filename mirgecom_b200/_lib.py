@@ -103,6 +103,7 @@ _SIGNATURES = {
                        C.c_size_t, _P, _P, _P], C.c_int),
     "mgc_rhs_split_f32": ([C.c_int, _P, _P, _P, _P, _P, _P, _P, C.c_int, C.c_int, _P, _P,
                            C.c_size_t, _P, _P, _P], C.c_int),
+    "mgc_rhs_hex": ([C.c_int, _P, _P, _P, _P, C.c_int, _P, _P, C.c_size_t, _P, _P, _P], C.c_int),
     "mgc_mlp_nparams": ([], C.c_int),
     "mgc_mlp_refresh": ([_P, _P], C.c_int),
     "mgc_mlp_infer": ([C.c_int, C.c_int, C.c_int64, _P, _P, _P, _P], C.c_int),

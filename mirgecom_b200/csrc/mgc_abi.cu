@@ -42,6 +42,8 @@ int tuh_upload_hexops(const double*);
 int tuhf_upload_hexops(const double*);
 int tuh_dispatch(int, int, int, bool, const DGArgs<double>&, const GasParams&, cudaStream_t);
 int tuhf_dispatch(int, int, int, bool, const DGArgs<float>&, const GasParams&, cudaStream_t);
+int tuh_rhs(int, bool, const DGArgs<double>&, const GasParams&, char*, cudaStream_t);
+size_t tuh_rhs_workspace(int, int64_t, int64_t);
 size_t tuh_split_workspace(int, int, bool, int64_t);
 size_t tuhf_split_workspace(int, int, bool, int64_t);
 }  // namespace mgc
@@ -338,7 +340,34 @@ int mgc_operator_f32(int viscous, const mgc_mesh_t* mesh, const mgc_gas_t* gas, 
 size_t mgc_rhs_split_workspace_bytes(const mgc_mesh_t* mesh, const mgc_gas_t* gas,
                                      int single_precision) {
   if (!mesh_ok(mesh) || !gas_ok(gas)) return 0;
-  return single_precision ? split_ws<float>(mesh, gas) : split_ws<double>(mesh, gas);
+  if (single_precision) return split_ws<float>(mesh, gas);
+  const size_t need = split_ws<double>(mesh, gas);
+  if (need == 0 || mesh->elem_kind != kElemHex) return need;
+  // mgc_rhs_hex uses the same buffer
+  const size_t hex = tuh_rhs_workspace(mesh->order, mesh->nelem, mesh->nbf);
+  return hex > need ? hex : need;
+}
+
+int mgc_rhs_hex(int viscous, const mgc_mesh_t* mesh, const mgc_gas_t* gas, const double* q,
+                const double* bext, int flux_kind, double* rhs, void* workspace,
+                size_t workspace_bytes, int32_t* status, void* stream, void* mid_event) {
+  if (!mesh_ok(mesh) || !gas_ok(gas) || !q || !rhs || !status || !workspace)
+    return MGC_E_INVALID;
+  if (flux_kind < 0 || flux_kind > 2) return MGC_E_INVALID;
+  if (mesh->elem_kind != kElemHex || gas->eos_kind != MGC_EOS_IDEAL || gas->nspecies != 0)
+    return MGC_E_UNSUPPORTED;
+  if (!mesh->fslot) return MGC_E_INVALID;
+  if (reinterpret_cast<uintptr_t>(workspace) % 256) return MGC_E_INVALID;
+  const int rc = ready(mesh, gas);
+  if (rc) return rc;
+  if (workspace_bytes < tuh_rhs_workspace(mesh->order, mesh->nelem, mesh->nbf))
+    return MGC_E_INVALID;
+  DGArgs<double> a = make_args<double>(mesh, q, nullptr, nullptr, nullptr, rhs, bext, flux_kind, 0,
+                                       status);
+  a.fslot = mesh->fslot;
+  a.mid_event = mid_event;
+  return tuh_rhs(mesh->order, viscous != 0, a, to_params(gas), static_cast<char*>(workspace),
+                 (cudaStream_t)stream);
 }
 
 int mgc_rhs_split(int viscous, const mgc_mesh_t* mesh, const mgc_gas_t* gas, const double* q,

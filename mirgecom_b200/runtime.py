@@ -308,7 +308,7 @@ def _split_workspace(dd, gs, f32):
     nbytes = lib.mgc_rhs_split_workspace_bytes(C.byref(dd.mesh), C.byref(gs), int(f32))
     if nbytes == 0:
         raise RuntimeError("split right-hand side unsupported for this configuration")
-    return dd.workspace("split_ws", ((nbytes + 15) // 16 * 16,), torch.uint8)
+    return dd.workspace("split_ws", ((nbytes + 255) // 256 * 256,), torch.uint8)
 
 
 def _operator_workspace(dd, gs, f32):
@@ -356,6 +356,20 @@ def _run_operator(viscous, dd, gs, q, t_op, t_src, bext, flux_kind, add_src, rhs
         events[2].record()
 
 
+def _hex_rhs_applies(dcoll, f32):
+    """The two-kernel right-hand side of hexahedra (mgc_rhs_hex): float64 (the
+    mixed form keeps the split passes and their roundings)."""
+    return dcoll.refel.kind == "hypercube" and not f32
+
+
+def _run_hex(viscous, dd, gs, q, bext, flux_kind, rhs, mid_event=None):
+    ws = _split_workspace(dd, gs, False)
+    _lib.check(_lib.load().mgc_rhs_hex(
+        int(viscous), C.byref(dd.mesh), C.byref(gs), _lib.ptr(q), _lib.ptr(bext), flux_kind,
+        _lib.ptr(rhs), _lib.ptr(ws), ws.numel(), _lib.ptr(dd.status), _lib.stream_handle(),
+        mid_event), "mgc_rhs_hex")
+
+
 def euler_rhs(dcoll, state, gas_model, boundaries, time, flux_kind):
     q = state.cv.q
     _lib.require_cuda(q)
@@ -380,6 +394,8 @@ def euler_rhs(dcoll, state, gas_model, boundaries, time, flux_kind):
         if _operator_path(path):
             _run_operator(False, dd, gs, q, t_op, None, bext, flux_kind, False, rhs, None,
                           phases=3 | (4 if path == "gradient_volume_face" else 0))
+        elif _hex_rhs_applies(dcoll, f32):
+            _run_hex(False, dd, gs, q, bext, flux_kind, rhs)
         elif path == "split":
             ws = _split_workspace(dd, gs, f32)
             fsplit = lib.mgc_rhs_split_f32 if f32 else lib.mgc_rhs_split
@@ -488,6 +504,17 @@ def ns_rhs(dcoll, state, gas_model, boundaries, time, flux_kind, *,
         if three and want_gradients:
             grad = grad.clone()
         return rhs, (grad if want_gradients else None)
+    if _hex_rhs_applies(dcoll, f32) and not want_gradients:
+        # no gradient pass: the volume kernel keeps the gradients on chip
+        with torch.cuda.device(q.device):
+            if events:
+                for ev in events[:-1]:
+                    ev.record()
+            _run_hex(True, dd, gs, q, bext, flux_kind, rhs,
+                     events[2].cuda_event if events and len(events) == 4 else None)
+            if events:
+                events[-1].record()
+        return rhs, None
     grad = dd.workspace("grad", gshape, q.dtype)
     fgrad = lib.mgc_ns_grad_f32 if f32 else lib.mgc_ns_grad
     frhs = lib.mgc_ns_rhs_f32 if f32 else lib.mgc_ns_rhs
