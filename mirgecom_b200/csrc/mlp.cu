@@ -17,8 +17,8 @@
 //
 // Training is three launches per step: forward + backward to the pre-
 // activation gradients (k_mlp_fwd_bwd, which also reduces the bias and
-// output-layer gradients), the weight gradients as split-K products over
-// the samples (k_mlp_wgrad), and Adam (k_mlp_adam).
+// output-layer gradients), the weight gradients of both layers as split-K
+// products over the samples (k_mlp_wgrad), and Adam (k_mlp_adam).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -93,15 +93,29 @@ struct Net {
   float out_shift, out_scale;
 };
 
+// [rows][W] bf16 in global memory to shared rows of stride WS, in 16-byte
+// pieces where the source allows it (single values took the training kernel
+// more instructions than its samples: 65,536 samples 44 -> 22 us, with one
+// round of resident blocks).
+template <int W, int WS>
+__device__ __forceinline__ void stage_rows(const __nv_bfloat16* src, __nv_bfloat16* dst, int rows) {
+  static_assert(W % 8 == 0 && WS % 8 == 0, "16-byte rows");
+  if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+    for (int i = threadIdx.x; i < rows * (W / 8); i += blockDim.x)
+      *reinterpret_cast<uint4*>(dst + (i / (W / 8)) * WS + i % (W / 8) * 8) =
+          reinterpret_cast<const uint4*>(src)[i];
+  } else {
+    for (int i = threadIdx.x; i < rows * W; i += blockDim.x) dst[(i / W) * WS + i % W] = src[i];
+  }
+}
+
 // Stage the bf16 weights in shared memory with padded rows.
 __device__ __forceinline__ void stage_weights(const Net& net, __nv_bfloat16* w1s,
                                               __nv_bfloat16* w2s, __nv_bfloat16* w2ts,
                                               float* /*bias*/) {
-  for (int i = threadIdx.x; i < H * KIN; i += blockDim.x) w1s[(i / KIN) * (KIN + 8) + i % KIN] = net.w1[i];
-  for (int i = threadIdx.x; i < H * H; i += blockDim.x) {
-    w2s[(i / H) * W2S + i % H] = net.w2[i];
-    if (w2ts) w2ts[(i / H) * W2S + i % H] = net.w2t[i];
-  }
+  stage_rows<KIN, KIN + 8>(net.w1, w1s, H);
+  stage_rows<H, W2S>(net.w2, w2s, H);
+  if (w2ts) stage_rows<H, W2S>(net.w2t, w2ts, H);
 }
 
 // bias layout in shared memory: [0,H) b1, [H,2H) b2, [2H,3H) w3, [3H] b3
@@ -301,7 +315,9 @@ __global__ void __launch_bounds__(WARPS * 32) k_mlp_infer(int64_t n, const float
 // x: [n][8] normalised inputs, tgt: [n] normalised targets.
 // Writes xb [n][KIN] (bf16 inputs), h1b [n][H] (bf16), dz1 / dz2 [n][H]
 // (bf16) and accumulates the gradients of b1, b2, w3, b3 and the loss sum.
-__global__ void __launch_bounds__(WARPS * 32) k_mlp_fwd_bwd(
+constexpr int kTrainBlocks = 3;      // per SM
+__host__ __device__ constexpr int imin_(int a, int b) { return a < b ? a : b; }
+__global__ void __launch_bounds__(WARPS * 32, kTrainBlocks) k_mlp_fwd_bwd(
     int64_t n, const float* __restrict__ x, const float* __restrict__ tgt, Net net,
     __nv_bfloat16* __restrict__ xb, __nv_bfloat16* __restrict__ h1b,
     __nv_bfloat16* __restrict__ dz1b, __nv_bfloat16* __restrict__ dz2b,
@@ -438,55 +454,114 @@ __global__ void __launch_bounds__(WARPS * 32) k_mlp_fwd_bwd(
   }
 }
 
-// dW[o][i] += sum_s dz[s][o] a[s][i]  (o < H, i < KA), split over samples.
-// Each warp owns one 16-row m-tile of o; a chunk of 16 samples is one k-step.
-template <int KA>
-__global__ void __launch_bounds__(WARPS * 32) k_mlp_wgrad(int64_t n,
-                                                          const __nv_bfloat16* __restrict__ dz,
-                                                          const __nv_bfloat16* __restrict__ a,
-                                                          float* __restrict__ dw) {
-  __shared__ __align__(16) __nv_bfloat16 dzt[H][16 + 8];   // [o][s]
-  __shared__ __align__(16) __nv_bfloat16 at[KA][16 + 8];   // [i][s]
+// A fragment (m16 x k16) and B fragments (k16 x 2 n8) of the bf16 product from
+// tiles stored [k][m] and [k][n]: 8x8 blocks read transposed.
+__device__ __forceinline__ void ldsm_trans(uint32_t (&v)[4], const __nv_bfloat16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+               : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+
+__device__ __forceinline__ void add_pair(float* p, float x, float y) {
+  if ((reinterpret_cast<uintptr_t>(p) & 7) == 0) {
+    atomicAdd(reinterpret_cast<float2*>(p), make_float2(x, y));
+  } else {
+    atomicAdd(p, x);
+    atomicAdd(p + 1, y);
+  }
+}
+
+// Weight gradients dW2[o][i] += sum_s dz2[s][o] h1[s][i] and dW1[o][i] +=
+// sum_s dz1[s][o] x[s][i], split over the samples: a block takes chunks of CH
+// samples, staged row by row (16-byte loads, the next chunk's in registers
+// while this one is contracted) and read transposed by ldmatrix; warp w owns
+// rows 16 w of both.  Two blocks per SM: with more, the final float atomics
+// (5120 per block) cost more than the products.  65,536 samples: 51 us in two
+// kernels that transposed by single bf16 stores, 10 us here.
+constexpr int CH = 64;
+__global__ void __launch_bounds__(WARPS * 32) k_mlp_wgrad(
+    int64_t n, const __nv_bfloat16* __restrict__ dz2, const __nv_bfloat16* __restrict__ h1,
+    const __nv_bfloat16* __restrict__ dz1, const __nv_bfloat16* __restrict__ x,
+    float* __restrict__ dw2, float* __restrict__ dw1) {
+  constexpr int XS = KIN + 8, NT = WARPS * 32;
+  __shared__ __align__(16) __nv_bfloat16 t_s[3][CH * W2S];   // dz2, h1, dz1
+  __shared__ __align__(16) __nv_bfloat16 x_s[CH * XS];
+  constexpr int RV = CH * H / 8 / NT, RX = CH * KIN / 8 / NT;  // uint4 per thread
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  constexpr int NT = KA / 8;
-  float acc[NT][4];
+  uint4 v[3][RV], vx[RX];
+  auto load = [&](int64_t ch) {
+    const uint4 zero = make_uint4(0, 0, 0, 0);
 #pragma unroll
-  for (int j = 0; j < NT; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
-  const int64_t nchunks = (n + 15) / 16;
-  for (int64_t ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < 16 * H; i += blockDim.x) {
-      const int s = i / H, o = i % H;
-      const int64_t gs = ch * 16 + s;
-      dzt[o][s] = gs < n ? dz[gs * H + o] : __float2bfloat16(0.f);
+    for (int j = 0; j < RV; ++j) {
+      const int i = threadIdx.x + j * NT;
+      const bool in = ch * CH + i / (H / 8) < n;
+      const int64_t o = ch * (CH * H / 8) + i;
+      v[0][j] = in ? reinterpret_cast<const uint4*>(dz2)[o] : zero;
+      v[1][j] = in ? reinterpret_cast<const uint4*>(h1)[o] : zero;
+      v[2][j] = in ? reinterpret_cast<const uint4*>(dz1)[o] : zero;
     }
-    for (int i = threadIdx.x; i < 16 * KA; i += blockDim.x) {
-      const int s = i / KA, c = i % KA;
-      const int64_t gs = ch * 16 + s;
-      at[c][s] = gs < n ? a[gs * KA + c] : __float2bfloat16(0.f);
-    }
-    __syncthreads();
-    // A[m=o][k=s] = dz^T, B[k=s][n=i] = a
-    const int o0 = warp * 16;
-    const uint32_t a0 = *reinterpret_cast<const uint32_t*>(&dzt[o0 + g][2 * t]);
-    const uint32_t a1 = *reinterpret_cast<const uint32_t*>(&dzt[o0 + g + 8][2 * t]);
-    const uint32_t a2 = *reinterpret_cast<const uint32_t*>(&dzt[o0 + g][2 * t + 8]);
-    const uint32_t a3 = *reinterpret_cast<const uint32_t*>(&dzt[o0 + g + 8][2 * t + 8]);
 #pragma unroll
-    for (int j = 0; j < NT; ++j) {
-      const uint32_t b0 = *reinterpret_cast<const uint32_t*>(&at[j * 8 + g][2 * t]);
-      const uint32_t b1 = *reinterpret_cast<const uint32_t*>(&at[j * 8 + g][2 * t + 8]);
-      mma_bf16(acc[j], a0, a1, a2, a3, b0, b1);
+    for (int j = 0; j < RX; ++j) {
+      const int i = threadIdx.x + j * NT;
+      vx[j] = ch * CH + i / (KIN / 8) < n ? reinterpret_cast<const uint4*>(x)[ch * (CH * KIN / 8) + i]
+                                          : zero;
+    }
+  };
+  float a2[8][4], a1[2][4];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) a2[j][0] = a2[j][1] = a2[j][2] = a2[j][3] = 0.f;
+#pragma unroll
+  for (int j = 0; j < 2; ++j) a1[j][0] = a1[j][1] = a1[j][2] = a1[j][3] = 0.f;
+  const int o0 = warp * 16;
+  const int blk = lane >> 3, row = lane & 7;
+  const int64_t nch = (n + CH - 1) / CH;
+  if ((int64_t)blockIdx.x < nch) load(blockIdx.x);
+  for (int64_t ch = blockIdx.x; ch < nch; ch += gridDim.x) {
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < RV; ++j) {
+      const int i = threadIdx.x + j * NT, o = i / (H / 8) * W2S + i % (H / 8) * 8;
+#pragma unroll
+      for (int m = 0; m < 3; ++m) *reinterpret_cast<uint4*>(&t_s[m][o]) = v[m][j];
+    }
+#pragma unroll
+    for (int j = 0; j < RX; ++j) {
+      const int i = threadIdx.x + j * NT;
+      *reinterpret_cast<uint4*>(&x_s[i / (KIN / 8) * XS + i % (KIN / 8) * 8]) = vx[j];
+    }
+    __syncthreads();
+    if (ch + gridDim.x < nch) load(ch + gridDim.x);
+#pragma unroll
+    for (int ks = 0; ks < CH; ks += 16) {
+      // A blocks (m, k), (m + 8, k), (m, k + 8), (m + 8, k + 8)
+      const int ao = (ks + (blk >> 1) * 8 + row) * W2S + o0 + (blk & 1) * 8;
+      uint32_t f2[4], f1[4], b[4];
+      ldsm_trans(f2, &t_s[0][ao]);
+      ldsm_trans(f1, &t_s[2][ao]);
+      // B blocks (k, n), (k + 8, n), (k, n + 8), (k + 8, n + 8)
+      const int kr = ks + (blk & 1) * 8 + row, nc = (blk >> 1) * 8;
+#pragma unroll
+      for (int j = 0; j < 8; j += 2) {
+        ldsm_trans(b, &t_s[1][kr * W2S + j * 8 + nc]);
+        mma_bf16(a2[j], f2[0], f2[1], f2[2], f2[3], b[0], b[1]);
+        mma_bf16(a2[j + 1], f2[0], f2[1], f2[2], f2[3], b[2], b[3]);
+      }
+      ldsm_trans(b, &x_s[kr * XS + nc]);
+      mma_bf16(a1[0], f1[0], f1[1], f1[2], f1[3], b[0], b[1]);
+      mma_bf16(a1[1], f1[0], f1[1], f1[2], f1[3], b[2], b[3]);
     }
   }
-  const int o0 = warp * 16;
 #pragma unroll
-  for (int j = 0; j < NT; ++j) {
-    const int c0 = j * 8 + 2 * t;
-    atomicAdd(&dw[(o0 + g) * KA + c0], acc[j][0]);
-    atomicAdd(&dw[(o0 + g) * KA + c0 + 1], acc[j][1]);
-    atomicAdd(&dw[(o0 + g + 8) * KA + c0], acc[j][2]);
-    atomicAdd(&dw[(o0 + g + 8) * KA + c0 + 1], acc[j][3]);
+  for (int j = 0; j < 8; ++j) {
+    const int c = j * 8 + 2 * t;
+    add_pair(&dw2[(o0 + g) * H + c], a2[j][0], a2[j][1]);
+    add_pair(&dw2[(o0 + g + 8) * H + c], a2[j][2], a2[j][3]);
+  }
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const int c = j * 8 + 2 * t;
+    add_pair(&dw1[(o0 + g) * KIN + c], a1[j][0], a1[j][1]);
+    add_pair(&dw1[(o0 + g + 8) * KIN + c], a1[j][2], a1[j][3]);
   }
 }
 
@@ -718,19 +793,22 @@ int mgc_mlp_train_grad(int64_t n, const float* x, const float* target, const mgc
     return MGC_E_INVALID;
   if (workspace_bytes < mgc_mlp_train_workspace_bytes(n)) return MGC_E_INVALID;
   cudaStream_t s = (cudaStream_t)stream;
-  __nv_bfloat16* xb = static_cast<__nv_bfloat16*>(workspace);
+  // 16-byte rows: the workspace's 256 spare bytes cover the alignment
+  __nv_bfloat16* xb = reinterpret_cast<__nv_bfloat16*>(
+      (reinterpret_cast<uintptr_t>(workspace) + 15) & ~uintptr_t(15));
   __nv_bfloat16* h1b = xb + (size_t)n * KIN;
   __nv_bfloat16* dz1b = h1b + (size_t)n * H;
   __nv_bfloat16* dz2b = dz1b + (size_t)n * H;
   if (cudaMemsetAsync(grad, 0, NPARAM * sizeof(float), s) != cudaSuccess) return MGC_E_CUDA;
   if (cudaMemsetAsync(loss, 0, sizeof(float), s) != cudaSuccess) return MGC_E_CUDA;
   const Net net = make_net(w);
-  const int nb = grid_for((n + 15) / 16);
+  // resident blocks only: each stages the weights once for its tiles
+  const int nb = imin_(grid_for((n + 15) / 16), 148 * kTrainBlocks);
   k_mlp_fwd_bwd<<<nb, WARPS * 32, 0, s>>>(n, x, target, net, xb, h1b, dz1b, dz2b, grad, loss,
                                          1.0f / (float)n);
-  const int nbw = (int)((n + 15) / 16 < 148 * 4 ? (n + 15) / 16 : 148 * 4);
-  k_mlp_wgrad<H><<<nbw, WARPS * 32, 0, s>>>(n, dz2b, h1b, grad + P_W2);
-  k_mlp_wgrad<KIN><<<nbw, WARPS * 32, 0, s>>>(n, dz1b, xb, grad + P_W1);
+  const int64_t nch = (n + CH - 1) / CH;
+  const int nbw = (int)(nch < 148 * 2 ? nch : 148 * 2);
+  k_mlp_wgrad<<<nbw, WARPS * 32, 0, s>>>(n, dz2b, h1b, dz1b, xb, grad + P_W2, grad + P_W1);
   return cudaGetLastError() == cudaSuccess ? MGC_OK : MGC_E_CUDA;
 }
 
