@@ -144,11 +144,15 @@ struct VCfg {
   static constexpr int NCOL3 = round_up(NC * EPB3, 8);
 
   // ---- face kernel
-  // float32: 8-element tiles in six resident blocks per SM (the face pass is
-  // bound by its gathers' latency: 8.7 ms against 9.8 ms for four blocks of
-  // 16 elements at 80^3)
-  static constexpr int NT2 = 128;
-  static constexpr int MINB2 = TF32 ? 6 : 4;
+  // 8-element tiles (the face pass is bound by its gathers' latency: 8.7 ms
+  // against 9.8 ms for four blocks of 16 elements at 80^3, float32), in 24 or
+  // 25 resident warps.  160 threads where they take the tile's face nodes in
+  // whole rounds (order-3 tetrahedra: 320 in two; with 128 the third round is
+  // half empty, 64^3 float32 3.27 -> 3.10 ms); 128 elsewhere (order 2 in one
+  // round of 192: 0.50 -> 0.62 ms at 40^3, four blocks hide less latency than
+  // six)
+  static constexpr int NT2 = TF32 && (8 * NFN) % 160 == 0 ? 160 : 128;
+  static constexpr int MINB2 = TF32 ? 800 / NT2 : 4;
   static constexpr int KFR = round_up(NFN, KSTEP);
   static constexpr int KF = Tile<R>::stride(KFR);
   static constexpr int A_FACE = NAC * MP * KF;
