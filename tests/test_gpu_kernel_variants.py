@@ -1,0 +1,92 @@
+"""Edges of the right-hand-side kernels' variants.
+
+* tcgen05 gradients at order 2 (two row blocks of eight elements, rows moved
+  in 8-byte pieces), against the mma.sync kernel and the float64 gradients,
+  as test_gpu_grad_tc.py does for orders 1 and 3;
+* the flux-volume kernel's staged inputs: rows off 16-byte boundaries are
+  copied by the threads instead of bulk copies, with identical results;
+* the mixture temperature from one polynomial pair per node against the
+  species sums (which mechanisms with differing mid temperatures take), with
+  iterations that cross the mid temperature.
+"""
+
+import copy
+
+import numpy as np
+import pytest
+import torch
+
+from cases import make_disc
+from mirgecom_b200 import runtime
+from mirgecom_b200.eos import PyrometheusMixture
+from mirgecom_b200.fluid import ConservedVars
+from mirgecom_b200.gas_model import GasModel, make_fluid_state
+from mirgecom_b200.initializers import reacting_mixture_state
+from mirgecom_b200.navierstokes import ns_operator
+from mirgecom_b200.thermochemistry import UIUC_7SP
+from mirgecom_b200.transport import SimpleTransport
+from test_gpu_grad_tc import _check, _mixture
+
+pytestmark = pytest.mark.gpu
+
+BOX = (0.02, 0.014, 0.026)
+
+
+def _gas(mech=UIUC_7SP):
+    return GasModel(eos=PyrometheusMixture(mech, temperature_niter=5),
+                    transport=SimpleTransport(viscosity=2e-5, thermal_conductivity=3e-2,
+                                              species_diffusivity=[1e-5] * 7))
+
+
+@pytest.mark.parametrize("n", [3, 5])
+def test_gradient_tc_order2(cuda, n):
+    d, od = make_disc("simplex", 3, n, 2, (0.0,) * 3, BOX, True)
+    gas, st64, st32 = _mixture(d, od, cuda, BOX, seed=n)
+    _check(d, gas, st64, st32, {}, min(BOX) / n)
+
+
+def _offset_copy(t):
+    """The same values one element past a 16-byte boundary."""
+    buf = torch.empty(t.numel() + 2, dtype=t.dtype, device=t.device)
+    out = buf[1:1 + t.numel()].view(t.shape)
+    out.copy_(t)
+    assert out.data_ptr() % 16 != 0
+    return out
+
+
+@pytest.mark.parametrize("dim,order", [(2, 1), (2, 3), (3, 1), (3, 2), (3, 3)])
+def test_flux_rows_off_16_bytes(cuda, dim, order):
+    d, od = make_disc("simplex", dim, 3, order, (0.0,) * dim, BOX[:dim], True)
+    cv0, t = reacting_mixture_state([torch.from_numpy(od.nodes[i]) for i in range(dim)], UIUC_7SP,
+                                    seed=2, t_range=(900.0, 1500.0), box=BOX[:dim])
+    gas = _gas()
+    out = []
+    for place in (lambda x: x, _offset_copy):
+        cv = ConservedVars(place(cv0.q.to(cuda)), dim)
+        st = make_fluid_state(cv, gas, temperature_seed=(t + 3.0).to(cuda))
+        out.append(ns_operator(d, gas, st, {}, species_source_temperature=st.temperature).q)
+    assert runtime.read_status(d) == 0
+    assert torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float64, 1e-12), (torch.float32, 2e-7)])
+def test_temperature_polynomial_against_species_sums(cuda, dtype, tol):
+    """1e-12: a hundred float64 roundings of energy terms up to ~50 c_v T;
+    2e-7: the float32 temperature's last two bits."""
+    g = torch.Generator().manual_seed(4)
+    n = 4099
+    x = [torch.rand(n, generator=g, dtype=torch.float64) * b for b in BOX]
+    cv0, t = reacting_mixture_state(x, UIUC_7SP, seed=3, box=BOX)
+    assert bool((t < 990).any()) and bool((t > 1010).any())
+    # seeds on the other side of the mid temperature (1000 K) for many nodes
+    seed = (t + 400.0 * (torch.rand(n, generator=g, dtype=torch.float64) - 0.5)).clamp(300, 2500)
+    other = copy.deepcopy(UIUC_7SP)
+    other.t_mid = UIUC_7SP.t_mid.copy()
+    other.t_mid[-1] += 1e-9
+    res = []
+    for mech in (UIUC_7SP, other):
+        gas = GasModel(eos=PyrometheusMixture(mech, temperature_niter=12))
+        st = make_fluid_state(ConservedVars(cv0.q.to(cuda, dtype).contiguous(), 3), gas,
+                              temperature_seed=seed.to(cuda, dtype))
+        res.append(st.temperature.double().cpu().numpy())
+    assert np.max(np.abs(res[0] - res[1]) / res[1]) < tol
