@@ -169,6 +169,8 @@ def stream_handle(device=None):
 
 def require_cuda(t):
     import torch
+    if t.is_cuda:
+        return
     if not torch.cuda.is_available():
         raise RuntimeError("mirgecom_b200 needs a CUDA device: no CPU fallback exists")
     if not t.is_cuda:

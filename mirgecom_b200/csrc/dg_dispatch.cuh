@@ -5,6 +5,10 @@
 #include <cuda_runtime.h>
 
 #include <cstring>
+#include <map>
+#include <mutex>
+#include <tuple>
+#include <utility>
 #include <vector>
 
 #include "dg_kernels.cuh"
@@ -110,12 +114,39 @@ inline int upload_mechanism_local(const Mechanism* m) {
   return cudaMemcpyToSymbol(c_mech32, &f, sizeof(f)) == cudaSuccess ? MGC_OK : MGC_E_CUDA;
 }
 
+// What the runtime has answered before for a kernel on a device: the largest
+// dynamic shared memory it allows so far, and the resident blocks for a block
+// size and shared memory (the attribute call and the occupancy query cost as
+// much as a launch).  A few entries per compiled kernel, shared by all
+// threads; if an entry cannot be kept (no memory) the question is asked again.
+struct LaunchCache {
+  std::mutex m;
+  std::map<std::pair<const void*, int>, size_t> smem;
+  std::map<std::tuple<const void*, int, int, size_t>, int64_t> blocks;
+};
+inline LaunchCache& launch_cache() {
+  static LaunchCache c;
+  return c;
+}
+
+// Allow *smem* bytes of dynamic shared memory (never lowered again: another
+// thread may be about to launch with more).
 template <class Kern>
 inline int prepare_kernel(Kern kern, size_t smem) {
-  if (smem > 48 * 1024) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-      return MGC_E_CUDA;
+  if (smem <= 48 * 1024) return MGC_OK;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return MGC_E_CUDA;
+  LaunchCache& c = launch_cache();
+  const std::pair<const void*, int> key{reinterpret_cast<const void*>(kern), dev};
+  std::lock_guard<std::mutex> lock(c.m);
+  const auto it = c.smem.find(key);
+  if (it != c.smem.end() && smem <= it->second) return MGC_OK;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+      cudaSuccess)
+    return MGC_E_CUDA;
+  try {
+    c.smem[key] = smem;
+  } catch (...) {
   }
   return MGC_OK;
 }
@@ -125,12 +156,29 @@ inline int prepare_kernel(Kern kern, size_t smem) {
 // capped at the number of work tiles.
 template <class Kern>
 inline int persistent_grid(Kern kern, int threads, size_t smem, int64_t tiles, int* nblk) {
-  int dev = 0, sms = 0, per_sm = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem) != cudaSuccess)
-    return MGC_E_CUDA;
-  int64_t nb = (int64_t)sms * (per_sm > 0 ? per_sm : 1);
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return MGC_E_CUDA;
+  LaunchCache& c = launch_cache();
+  const std::tuple<const void*, int, int, size_t> key{reinterpret_cast<const void*>(kern), dev,
+                                                      threads, smem};
+  int64_t nb = 0;
+  {
+    std::lock_guard<std::mutex> lock(c.m);
+    const auto it = c.blocks.find(key);
+    if (it != c.blocks.end()) nb = it->second;
+  }
+  if (nb == 0) {
+    int sms = 0, per_sm = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem) != cudaSuccess)
+      return MGC_E_CUDA;
+    nb = (int64_t)sms * (per_sm > 0 ? per_sm : 1);
+    std::lock_guard<std::mutex> lock(c.m);
+    try {
+      c.blocks[key] = nb;
+    } catch (...) {
+    }
+  }
   if (nb > tiles) nb = tiles;
   *nblk = (int)(nb > 0 ? nb : 1);
   return MGC_OK;

@@ -94,6 +94,7 @@ class DeviceDiscretization:
             dcoll.refel.face_nodes[c.bface_face].astype(np.int64)).to(device)
         self.status = torch.zeros(1, dtype=torch.int32, device=device)
         self._bkind_cache = {}
+        self._tag_cache = {}
         self._work = {}
         self.mesh = _lib.MeshStruct()
         self.mesh.dim = dcoll.dim
@@ -117,6 +118,26 @@ class DeviceDiscretization:
             t = torch.empty(shape, dtype=dtype, device=self.device)
             self._work[name] = t
         return t
+
+    def boundary_tag(self, tag):
+        """Device index data of the boundary faces under *tag*: their numbers
+        (None: every face, in order), elements [n, 1] and face-node volume
+        indices [n, Nfp], node coordinates (dim, n, Nfp) and unit normals
+        (dim, n, 1).  The mesh does not change, so they are uploaded once; a
+        boolean mask per call cost a device-to-host synchronisation per
+        indexing (the order-3 16 x 16 vortex step: 2.2 ms, 1.4 ms so)."""
+        key = str(tag)
+        if key not in self._tag_cache:
+            mask = self.dcoll.boundary_face_mask(tag)
+            idx = None if mask.all() else torch.from_numpy(np.nonzero(mask)[0]).to(self.device)
+            nrm = np.ascontiguousarray(self.dcoll.boundary_normals_numpy()[mask].T)
+            self._tag_cache[key] = (
+                idx,
+                (self.bface_elem if idx is None else self.bface_elem[idx])[:, None],
+                self.bface_nodes if idx is None else self.bface_nodes[idx],
+                self.dcoll.boundary_nodes(tag, self.device),
+                torch.from_numpy(nrm).to(self.device)[:, :, None])
+        return self._tag_cache[key]
 
     def bkind_for(self, boundaries):
         """int8 [nbf] boundary kinds for this *boundaries* dict."""
@@ -226,30 +247,24 @@ def boundary_exterior(dd, state, gas_model, boundaries, time):
     nc = q.shape[0]
     nfp = dcoll.nface_nodes
     bext = dd.workspace("bext", (nc + 1, dd.nbf, nfp), q.dtype)
-    be = dd.bface_elem[:, None]
-    qm = q[:, be, dd.bface_nodes]                          # [Nc, nbf, Nfp]
     from mirgecom_b200.fluid import ConservedVars
     from mirgecom_b200.gas_model import FluidState
-    tm = None
-    if state.is_mixture:
-        tm = state.temperature[be, dd.bface_nodes]
     for tag, bdry in boundaries.items():
         if not wants(bdry):
             continue
-        mask = torch.from_numpy(dcoll.boundary_face_mask(tag)).to(q.device)
-        sm = FluidState(ConservedVars(qm[:, mask], state.dim), gas_model,
-                        temperature=None if tm is None else tm[mask])
+        idx, be, bn, nodes, nrm = dd.boundary_tag(tag)
+        faces = slice(None) if idx is None else idx
+        sm = FluidState(ConservedVars(q[:, be, bn], state.dim), gas_model,
+                        temperature=state.temperature[be, bn] if state.is_mixture else None)
         if isinstance(bdry, MengaldoBoundaryCondition):
-            bext[:, mask] = bdry.exterior_parameters(dcoll, gas_model, sm, nc).to(q.dtype)
+            bext[:, faces] = bdry.exterior_parameters(dcoll, gas_model, sm, nc).to(q.dtype)
             continue
-        nrm = torch.from_numpy(np.ascontiguousarray(
-            dcoll.boundary_normals_numpy()[dcoll.boundary_face_mask(tag)].T)).to(q.device)
-        ext = bdry.exterior_state(dcoll, tag, gas_model, sm, time,
-                                  nodes=dcoll.boundary_nodes(tag, q.device),
-                                  normals=nrm[:, :, None])
-        bext[:nc, mask] = ext.cv.q.to(q.dtype)
+        # the callback gets its own coordinates, as from a fresh evaluation
+        ext = bdry.exterior_state(dcoll, tag, gas_model, sm, time, nodes=nodes.clone(),
+                                  normals=nrm)
+        bext[:nc, faces] = ext.cv.q.to(q.dtype)
         if state.is_mixture:
-            bext[nc, mask] = ext.temperature.to(q.dtype)
+            bext[nc, faces] = ext.temperature.to(q.dtype)
     return bext
 
 
