@@ -37,9 +37,10 @@
 //
 // Bound: the producers' gathers, latency and L1 wavefronts (the products are
 // 0.4 us of a 2.9 us tile).  Against the version with per-face lift columns
-// and no reload in place (CUDA events): order 3, 64^3 cells 4.38 -> 4.33 ms
-// (32^3: 232 M -> 160 M warp instructions), 1260 tetrahedra 17.2 -> 12.4 us;
-// order 2, 40^3 cells 745 us (799 us by k_grad, which it replaces there).
+// and no reload in place (CUDA events): order 3, 64^3 cells 4.38 -> 4.06 ms
+// (of it 0.27 by working out each thread's item indices once instead of per
+// tile), 1260 tetrahedra 17.2 -> 12.2 us; order 2, 40^3 cells 687 us (799 us
+// by k_grad, which it replaces there).
 //
 // Operands use the K-major, non-swizzled canonical layout of the UMMA
 // descriptors: 8-row x 16-byte core matrices, row groups SBO = 128 bytes
@@ -326,12 +327,33 @@ __global__ void __launch_bounds__(TcGrad<DIM, ORDER, NS>::NT, 1)
     VecF<VW> rv[RR];
     float nb[NU];
     int fmode = -1;
-    auto row_load = [&](int tl, int j) {
+    // this thread's row pieces (the same in every tile): source in element 0's
+    // tile, and packed: operand offset in the stage | index of the row's shift
+    // | element (63: none).  Worked out per tile, with 64-bit sums per load,
+    // the indices were half of the producers' instructions.
+    const float* rsrc[RR];
+    uint32_t rpk[RR];
+    static_assert(C::STAGE <= 1 << 17 && NU * EPB <= 512 && EPB < 63, "packed row items");
+#pragma unroll
+    for (int j = 0; j < RR; ++j) {
       const int idx = tid + j * GT;
       const int kc = idx % (NP / VW), e = (idx / (NP / VW)) % EPB, c = idx / (NP / VW * EPB);
-      if (idx < C::ROW_ITEMS && tl * EPB + e < EOWN)
-        rv[j].load(field(c) + (int64_t)(tl * EPB + e) * NP + kc * VW);
+      const bool in = idx < C::ROW_ITEMS;
+      rsrc[j] = field(in ? c : 0) + e * NP + kc * VW;
+      rpk[j] = in ? (uint32_t)(2 * (e / EPM) * C::A_BYTES + canon_off(c * EPM + e % EPM, kc * VW, C::LBO_A)) |
+                        (uint32_t)(c * EPB + e) << 17 | (uint32_t)e << 26
+                  : 63u << 26;
+    }
+    auto row_load = [&](int tl, int j) {
+      const int e = (int)(rpk[j] >> 26);
+      if (e < EOWN - tl * EPB && e != 63) rv[j].load(rsrc[j] + (int64_t)tl * (EPB * NP));
     };
+    // the neighbour's fields at node *gi* (node numbers times four fit 32 bits)
+    auto face_load = [&](int64_t gi, int c) {
+      return __ldg(reinterpret_cast<const float*>(reinterpret_cast<const char*>(field(c)) +
+                                                  (uint32_t)gi * 4u));
+    };
+    const int foff = 2 * (fe / EPM) * C::A_BYTES + canon_off(fe % EPM, KV + ffm, C::LBO_A);
     // mode of this thread's face node in tile tl (pairing words *conn_b*):
     // -1 none, 0 interior (en, kn its neighbour node), 1 exterior value,
     // 2 interior value, 3 Mengaldo
@@ -415,7 +437,7 @@ __global__ void __launch_bounds__(TcGrad<DIM, ORDER, NS>::NT, 1)
       fmode = face_mode(first, small_s, gi);
       if (fmode == 0) {
 #pragma unroll
-        for (int c = 0; c < NU; ++c) nb[c] = __ldg(field(c) + gi);
+        for (int c = 0; c < NU; ++c) nb[c] = face_load(gi, c);
       }
     }
     for (int it = 0, tile = first, b = 0; tile < ntiles; ++it, tile += step) {
@@ -452,15 +474,12 @@ __global__ void __launch_bounds__(TcGrad<DIM, ORDER, NS>::NT, 1)
       // ---- rows: shift, split, store; reload for the next tile
 #pragma unroll
       for (int j = 0; j < RR; ++j) {
-        const int idx = tid + j * GT;
-        const int kc = idx % (NP / VW), e = (idx / (NP / VW)) % EPB, c = idx / (NP / VW * EPB);
-        if (idx < C::ROW_ITEMS && e < ne) {
+        if ((int)(rpk[j] >> 26) < ne) {
           VecF<VW> h, l;
-          rv[j].shift_split(u0_b[c * EPB + e], h, l);
-          unsigned char* blk = stage + 2 * (e / EPM) * C::A_BYTES;
-          const int o = canon_off(c * EPM + e % EPM, kc * VW, C::LBO_A);
-          h.store(reinterpret_cast<float*>(blk + o));
-          l.store(reinterpret_cast<float*>(blk + C::A_BYTES + o));
+          rv[j].shift_split(u0_b[rpk[j] >> 17 & 511], h, l);
+          unsigned char* dst = stage + (rpk[j] & 0x1ffff);
+          h.store(reinterpret_cast<float*>(dst));
+          l.store(reinterpret_cast<float*>(dst + C::A_BYTES));
         }
         if (more) row_load(tile + step, j);
       }
@@ -471,14 +490,13 @@ __global__ void __launch_bounds__(TcGrad<DIM, ORDER, NS>::NT, 1)
       if (more) fmode = face_mode(tile + step, small_s + bn * C::SMALL, gn);
       const bool reload = more && fmode == 0;
       if (mode >= 0) {
-        unsigned char* fdst = stage + 2 * (fe / EPM) * C::A_BYTES +
-                              canon_off(fe % EPM, KV + ffm, C::LBO_A);
+        unsigned char* fdst = stage + foff;
         if (mode == 0) {
 #pragma unroll
           for (int c = 0; c < NU; ++c) {
             float hi, lo;
             split_f32((nb[c] - u0_b[c * EPB + fe]) * 0.5f, hi, lo);
-            if (reload) nb[c] = __ldg(field(c) + gn);
+            if (reload) nb[c] = face_load(gn, c);
             const int o = c * EPM * 16;
             *reinterpret_cast<float*>(fdst + o) = hi;
             *reinterpret_cast<float*>(fdst + o + C::A_BYTES) = lo;
@@ -521,7 +539,7 @@ __global__ void __launch_bounds__(TcGrad<DIM, ORDER, NS>::NT, 1)
       }
       if (mode != 0 && reload) {
 #pragma unroll
-        for (int c = 0; c < NU; ++c) nb[c] = __ldg(field(c) + gn);
+        for (int c = 0; c < NU; ++c) nb[c] = face_load(gn, c);
       }
       // ---- the epilogue's copy of the metric; per-tile data two tiles ahead
       // (into the buffer of the tile before this one)
