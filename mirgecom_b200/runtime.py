@@ -497,10 +497,14 @@ def ns_rhs(dcoll, state, gas_model, boundaries, time, flux_kind, *,
             grad = torch.empty(gshape, dtype=q.dtype, device=q.device) if want_gradients else None
         # three kernels: the gradient entry point (its own launch, timed by
         # events[0..1]), then the operator with the gradients given (bit 8)
-        extra = 4 | 8 if three else 0
+        # (one library call for all three when nothing is recorded or
+        # exchanged in between)
+        one_call = three and not events and halo is None and phases == 3 \
+            and getattr(dcoll, "nowned", None) is None
+        extra = 4 if one_call else 4 | 8 if three else 0
         ops_events = events[1:] if (events and three) else events
         with torch.cuda.device(q.device):
-            if three and (phases & 1):
+            if three and (phases & 1) and not one_call:
                 if events:
                     events[0].record()
                 fgrad = lib.mgc_ns_grad_f32 if f32 else lib.mgc_ns_grad
