@@ -1373,9 +1373,13 @@ __global__ void __launch_bounds__(256, (Cfg<R, DIM, ORDER, NS, MIX>::MINB_SURF))
   constexpr int NP = C::NP, NF = C::NF, NFP = C::NFP, NFN = C::NFN, NC = C::NC, FW = C::FW;
   constexpr int EPB = C::EPB_SURF, MP = C::MP, MT = C::MT, KB = C::KB, KR = C::KR;
   constexpr int KRR = C::KRR, NCOL = C::NCOL_S;
-  constexpr int CG = 4;                     // fields per work item
+  // fields per work item: all five of the 3-D ideal gas, so that a face node's
+  // gathers are one batch and every item has the same work (a group of 4 and one
+  // of 1 before: 24^3 p3 Taylor-Green, float64 372 -> 313 us); 4 elsewhere, where
+  // a node's record does not fit the registers
+  constexpr int CG = NC == 5 ? 5 : 4;
   constexpr int NG = (NC + CG - 1) / CG;    // field groups
-  constexpr int GV = CG * DIM;              // record values per group
+  constexpr int GV = round_up(CG * DIM, 4); // record values per group, whole loads
   constexpr int LIM = NC * DIM;             // end of the flux part of a record
   extern __shared__ __align__(16) unsigned char smem_raw[];
   R* am = reinterpret_cast<R*>(smem_raw);                  // [NAC][MP][KB]
