@@ -303,7 +303,11 @@ __global__ void __launch_bounds__(256, 2) k_hex_surface(DGArgs<R> a, GasParams g
   constexpr int N1 = H::N1, NP = H::NP, NFP = H::NFP, NFN = H::NFN, NL = H::NL;
   constexpr int NC = C::NC, EPB = C::EPB_S, DIM = 3;
   constexpr int FW = flux_record_width(DIM, NC);
-  constexpr int CG = 4, NG = (NC + CG - 1) / CG, GV = CG * DIM, LIM = NC * DIM;
+  // fields per work item: float32 takes all five of the ideal gas at once, so
+  // that a face node's gathers are one batch (48^3 p4: 2.37 -> 1.85 ms);
+  // float64 (reached only where the gradients are asked for) keeps groups of 4
+  constexpr int CG = NC == 5 && sizeof(R) == 4 ? 5 : 4, NG = (NC + CG - 1) / CG;
+  constexpr int GV = round_up(CG * DIM, 4), LIM = NC * DIM;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   R* g_s = reinterpret_cast<R*>(smem_raw);              // [EPB][NC][3][NP]
   R* s_s = g_s + EPB * NC * 3 * NP;                     // [EPB][NC][NF][NFP]
