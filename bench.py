@@ -138,7 +138,7 @@ def contraction_flops(dcoll, nc):
 
 KERNEL_NAMES = {"state": "k_mixture_state*", "grad": "k_grad*", "node_flux": "k_node_flux",
                 "surface": "k_surface", "volume": "k_volume", "flux_volume": "k_flux_volume",
-                "face": "k_face"}
+                "face": "k_face", "hex_volume": "k_hex_volume", "hex_face": "k_hex_face"}
 
 
 def algorithmic_bytes(dcoll, nc, s=8, mixture=False):
@@ -179,6 +179,10 @@ def algorithmic_bytes(dcoll, nc, s=8, mixture=False):
         "surface": nn * (fw + nc + (ns if mixture else 0) + nc) * s + geo,
         "rhs": nn * (nc + (nc + 1) * d + nc + 2 * t_in) * s + geo,
     }
+    # float64 hexahedra: the volume kernel writes each node's wave speed too,
+    # the face kernel reads it
+    out["hex_volume"] = out["volume"] + nn * s
+    out["hex_face"] = out["face"] + nn * s
     if mixture:
         out["state"] = nn * (nc + 1 + (2 if s == 8 else 1)) * s
     return out
@@ -426,6 +430,10 @@ def _time_form(dcoll, gas, q, tseed, steps, warmup, flush, stream):
     elif three:
         kern = {"state": mean(0, 1), "grad": mean(1, 2), "flux_volume": mean(2, 3),
                 "face": mean(3, 4), "rhs": mean(1, 4)}
+    elif runtime._hex_rhs_applies(dcoll, q.dtype == torch.float32):
+        # start | state | (no gradient pass) | volume | face
+        kern = {"state": mean(0, 1), "hex_volume": mean(2, 3), "hex_face": mean(3, 4),
+                "rhs": mean(2, 4)}
     else:
         kern = {"state": mean(0, 1), "grad": mean(1, 2), "node_flux": mean(2, 3),
                 "surface": mean(3, 4), "rhs": mean(2, 4)}

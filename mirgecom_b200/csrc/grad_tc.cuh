@@ -36,7 +36,7 @@
 // work in it.
 //
 // Bound: the producers' gathers, latency and L1 wavefronts (the products are
-// 0.4 us of a 2.9 us tile).  Against the version with per-face lift columns
+// 0.4 us of a 3.4 us tile).  Against the version with per-face lift columns
 // and no reload in place (CUDA events): order 3, 64^3 cells 4.38 -> 4.06 ms
 // (of it 0.27 by working out each thread's item indices once instead of per
 // tile), 1260 tetrahedra 17.2 -> 12.2 us; order 2, 40^3 cells 687 us (799 us

@@ -6,7 +6,8 @@ boundary fluxes, weak divergence, face lift and inverse mass -- runs on the
 device (``runtime.euler_rhs``): on simplicial meshes two kernels through
 ``mgc_operator`` (a volume kernel for the pointwise fluxes, face-node records
 and the volume part of the divergence, a face kernel for the numerical
-fluxes and the lift); on hexahedra the split divergence pass.
+fluxes and the lift); on hexahedra two kernels of the same kind through
+``mgc_rhs_hex`` in float64, the split divergence pass in float32.
 """
 
 from __future__ import annotations

@@ -5,7 +5,9 @@ div(F_V - F_I) with BR1 gradients on the device (``runtime.ns_rhs``): on
 simplicial meshes in two kernels through ``mgc_operator`` (a volume kernel
 that keeps the gradients on chip and evaluates the pointwise fluxes and the
 volume part of the divergence, and a face kernel for the numerical fluxes and
-the lift); on hexahedra as a gradient pass and a split divergence pass.
+the lift); on hexahedra as the same two kernels through ``mgc_rhs_hex`` in
+float64, as a gradient pass and a split divergence pass in float32 or where the
+gradients are asked for.
 For a reacting mixture the species source terms (the driver-side
 ``eos.get_species_source_terms`` of examples/gas-in-box.py:702-705) are
 fused into the volume kernel by passing ``species_source_temperature``.

@@ -296,7 +296,8 @@ def _operator_temperature(state):
 #                  kernel phases (partitions); "split" otherwise (the ideal gas
 #                  without walls: 0.55 ms against 0.585 ms for the 24^3 p3
 #                  Taylor-Green right-hand side)
-# Tensor-product hexahedra always take "split".
+# Tensor-product hexahedra take mgc_rhs_hex in float64 (two kernels, gradients
+# on chip) unless the caller wants the gradients, and "split" otherwise.
 RHS_PATH = "auto"
 
 
