@@ -471,6 +471,9 @@ def ns_rhs(dcoll, state, gas_model, boundaries, time, flux_kind, *,
     :func:`face_records` in between."""
     path = _path(dcoll, gas_model, boundaries, phased=(phases != 3 or halo is not None))
     _check_boundary_path(dcoll, boundaries, path)
+    if source_temperature is not None and not state.is_mixture:
+        # on every layout: mgc_rhs_hex has no argument for them to refuse
+        raise RuntimeError("species sources need a mixture equation of state")
     q = state.cv.q
     _lib.require_cuda(q)
     q = q.contiguous()

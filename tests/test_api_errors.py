@@ -81,3 +81,16 @@ def test_unsupported_options(case):
     vgas = GasModel(eos=IdealSingleGas(), transport=SimpleTransport(viscosity=1e-3))
     with pytest.raises(NotImplementedError):
         ns_operator(d, vgas, make_fluid_state(cv, vgas), {}, inviscid_terms_on=False)
+
+
+@pytest.mark.parametrize("kind,dim", [("hypercube", 3), ("simplex", 3), ("simplex", 2)])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+@pytest.mark.parametrize("gradients", [False, True])
+def test_species_sources_need_a_mixture(kind, dim, dtype, gradients):
+    """On every layout of the right-hand side, with and without gradients."""
+    d, od = make_disc(kind, dim, 3, 1, (0.0,) * dim, (1.0,) * dim, True)
+    cv = ConservedVars(torch.from_numpy(perturbed_state_np(od.nodes, dim, 0, seed=2)).to(dtype), dim)
+    gas = GasModel(eos=IdealSingleGas(), transport=SimpleTransport(viscosity=1e-3))
+    with pytest.raises(RuntimeError, match="mixture"):
+        ns_operator(d, gas, make_fluid_state(cv, gas), {}, return_gradients=gradients,
+                    species_source_temperature=torch.ones_like(cv.q[0]))
