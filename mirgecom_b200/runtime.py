@@ -259,9 +259,10 @@ def boundary_exterior(dd, state, gas_model, boundaries, time):
         if isinstance(bdry, MengaldoBoundaryCondition):
             bext[:, faces] = bdry.exterior_parameters(dcoll, gas_model, sm, nc).to(q.dtype)
             continue
-        # the callback gets its own coordinates, as from a fresh evaluation
+        # the callback gets its own coordinates and normals, as from a fresh
+        # evaluation
         ext = bdry.exterior_state(dcoll, tag, gas_model, sm, time, nodes=nodes.clone(),
-                                  normals=nrm)
+                                  normals=nrm.clone())
         bext[:nc, faces] = ext.cv.q.to(q.dtype)
         if state.is_mixture:
             bext[nc, faces] = ext.temperature.to(q.dtype)
