@@ -1,6 +1,7 @@
 """Boundary data handed to ``exterior_state`` (``runtime.boundary_exterior``):
 the coordinates and unit normals are the callee's own, a call that changes them
-in place changes no later call (host side, CPU tensors)."""
+in place changes no later call (host side, CPU tensors); and the data kept per
+tag are complete for every stream once they are kept (GPU)."""
 
 import numpy as np
 import pytest
@@ -52,3 +53,27 @@ def test_callbacks_own_their_nodes_and_normals(kind, dim, per_side):
         np.testing.assert_array_equal(nodes.numpy(), d.boundary_nodes_numpy()[:, mask])
         np.testing.assert_array_equal(normals[:, :, 0].numpy(),
                                       d.boundary_normals_numpy()[mask].T)
+
+
+@pytest.mark.gpu
+def test_tag_data_are_complete_for_other_streams(cuda):
+    """Kept while the first caller's stream is busy, read on another one."""
+    d, _ = make_disc("simplex", 3, 4, 2, (0.0,) * 3, (1.0, 0.8, 1.2), False)
+    dd = runtime.device_discretization(d, cuda)
+    torch.cuda.synchronize()
+    busy, other = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(busy):
+        torch.cuda._sleep(200_000_000)                     # about 0.1 s
+        for tag in TAGS:
+            dd.boundary_tag(tag)
+    c = d.connectivity
+    with torch.cuda.stream(other):
+        for tag in TAGS:
+            got = [v.cpu().numpy() for v in dd.boundary_tag(tag)]
+            mask = d.boundary_face_mask(tag)
+            want = (np.nonzero(mask)[0], c.bface_elem[mask][:, None],
+                    d.refel.face_nodes[c.bface_face[mask]], d.boundary_nodes_numpy()[:, mask],
+                    d.boundary_normals_numpy()[mask].T[:, :, None])
+            for g, w in zip(got, want):
+                np.testing.assert_array_equal(g, w)
+    torch.cuda.synchronize()
