@@ -19,6 +19,8 @@
 
 #include <cstring>
 
+#include "quotient.cuh"
+
 #define MGC_MAX_SPECIES 16
 #define MGC_MAX_REACTIONS 8
 
@@ -487,21 +489,16 @@ struct NodeState {
 // Fill the thermodynamic state.  For the ideal gas the temperature is
 // computed from q; for mixtures *t_in* is the converged temperature.
 //
-// Per-node quotients by the density, from its correctly rounded reciprocal
-// (one division per node instead of ~40 in the state and the viscous flux).
-// float32 multiplies (at most one more rounding per quotient); float64 adds
-// Markstein's correction step (P. Markstein, "Computation of elementary
-// functions on the IBM RISC System/6000 processor", 1990): with the residual
-// x - rho q exact in a fused multiply-add, q + irho (x - rho q) is the
-// correctly rounded quotient, in three instructions.  With the
-// square roots in conc_pow: flux-volume kernel, float64 32^3 p3, 2.46 -> 2.04 ms.
+// Per-node quotients by the density, from its reciprocal (one division per node
+// instead of ~40 in the state and the viscous flux).  float32 multiplies (at
+// most one more rounding per quotient); float64 takes the rounded quotient
+// (quotient.cuh).
 template <class R>
 __device__ __forceinline__ R per_rho(R x, R rho, R irho) {
-  const R q = x * irho;
   if constexpr (sizeof(R) == 4) {
-    return q;
+    return x * irho;
   } else {
-    return fma(fma(-rho, q, x), irho, q);
+    return quotient(x, rho, irho);
   }
 }
 
