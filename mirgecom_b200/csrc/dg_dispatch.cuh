@@ -254,6 +254,27 @@ struct Launch {
   static size_t split_workspace_bytes(int64_t nelem) {
     return ((size_t)nelem * C::NP * C::FW + (size_t)NS * nelem * C::NP) * sizeof(R) + 256;
   }
+  // every row of the flux-volume kernel's tiles starts on 16 bytes
+  template <bool VISC>
+  static bool flux_rows_aligned(const DGArgs<R>& a) {
+    auto at = [](const R* p) { return reinterpret_cast<uintptr_t>(p); };
+    const uintptr_t al = at(a.q) | (MIX ? at(a.t_op) : 0) |
+                         (MIX && a.add_sources ? at(a.t_src) : 0) | (VISC ? at(a.grad) : 0);
+    return (al & 15) == 0 && ((int64_t)a.nelem * C::NP * sizeof(R)) % 16 == 0;
+  }
+  template <bool VISC, bool STAGED>
+  static int flux_volume(const DGArgs<R>& a, const GasParams& g, cudaStream_t s) {
+    using V = VCfg<R, DIM, ORDER, NS, MIX>;
+    constexpr int EPB = V::epb3(STAGED);
+    const size_t smem = V::flux_bytes(EPB, VISC, STAGED);
+    auto kern = k_flux_volume<R, DIM, ORDER, NS, MIX, VISC, STAGED>;
+    int nblk = 0, rc = prepare_kernel(kern, smem);
+    if (rc) return rc;
+    rc = persistent_grid(kern, V::NT3, smem, (a.nowned + EPB - 1) / EPB, &nblk);
+    if (rc) return rc;
+    kern<<<nblk, V::NT3, smem, s>>>(a, g);
+    return cudaGetLastError() == cudaSuccess ? MGC_OK : MGC_E_CUDA;
+  }
   // volume kernel then face kernel (dg_volume.cuh)
   // a.phases: bit 0 the volume stage, bit 1 the face kernel; bit 2 runs the
   // volume stage as the gradient kernel (gradients into a.grad_out) and the
@@ -277,14 +298,9 @@ struct Launch {
         }
         b.grad = a.grad_out;
       }
-      const size_t smem3 = V::flux_bytes(V::EPB3, VISC);
-      auto k3 = k_flux_volume<R, DIM, ORDER, NS, MIX, VISC>;
-      rc = prepare_kernel(k3, smem3);
+      rc = flux_rows_aligned<VISC>(b) ? flux_volume<VISC, true>(b, g, s)
+                                      : flux_volume<VISC, false>(b, g, s);
       if (rc) return rc;
-      rc = persistent_grid(k3, V::NT3, smem3, (a.nowned + V::EPB3 - 1) / V::EPB3, &nblk);
-      if (rc) return rc;
-      k3<<<nblk, V::NT3, smem3, s>>>(b, g);
-      if (cudaGetLastError() != cudaSuccess) return MGC_E_CUDA;
     } else if (phases & 1) {
       const size_t smem1 = V::vol_bytes(V::EPB, a.nperm);
       auto k1 = k_volume<R, DIM, ORDER, NS, MIX, VISC>;

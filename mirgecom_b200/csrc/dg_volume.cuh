@@ -59,9 +59,6 @@ struct RecLayout {
   static __device__ __forceinline__ int chunk(int slot, int t) {
     return ROT ? ((t + slot / PER_LINE) & (NCH - 1)) * VEC : t * VEC;
   }
-  static __device__ __forceinline__ int at(int slot, int i) {
-    return chunk(slot, i / VEC) + i % VEC;
-  }
 };
 
 template <class R, int DIM, int ORDER, int NS, bool MIX>
@@ -114,8 +111,9 @@ struct VCfg {
 
   // ---- flux-volume kernel (gradients from HBM): no gradient operands or
   // staging of its own gradients; element tiles sized so the pointwise phase
-  // fills the block.  The tile's inputs are staged in shared memory: rows of
-  // the NC fields, the operator and source temperatures, the gradients
+  // fills the block.  Where the rows allow it (STAGED below) the tile's inputs
+  // are staged in shared memory: rows of the NC fields, the operator and source
+  // temperatures, the gradients
   static constexpr int NT3 = TF32 ? 256 : 128;
   // operator rows: NP per r.  The last m-tile reads up to MP rows, on into the
   // next matrix or gfl (accumulator rows >= NP, never stored)
@@ -126,22 +124,22 @@ struct VCfg {
   }
   static constexpr int GEO3 = DIM * DIM + NF * DIM;        // metric, unit normals
   static constexpr __host__ __device__ int nnode3(int epb) { return epb * NP + (KUR - NP) + 4; }
-  static constexpr __host__ __device__ size_t flux_bytes(int epb, bool visc) {
+  static constexpr __host__ __device__ size_t flux_bytes(int epb, bool visc, bool staged) {
     return (size_t)round_up(A_FLUX + nnode3(epb) * FST + NS * epb * NP + 2 * epb * GEO3 +
                                 epb * NC * DIM, 4) * RB +
-           (size_t)round_up(epb * NP * RB, 16) * rows3(visc) + NFN * 4 + 2 * epb * NF * 4 +
-           NP * NF * 2 + 64;
+           (staged ? (size_t)round_up(epb * NP * RB, 16) * rows3(visc) : 0) + NFN * 4 +
+           2 * epb * NF * 4 + NP * NF * 2 + 64;
   }
   // the largest tile with at most one node per thread and two blocks per SM;
-  // even, so that rows of NP even values start on 16 bytes
-  static constexpr __host__ __device__ int pick_epb3() {
+  // staged rows of a tile start on 16 bytes
+  static constexpr __host__ __device__ int epb3(bool staged) {
     int best = 1;
-    for (int e = 2; e * NP <= NT3; e += 2)
-      if (flux_bytes(e, true) <= (size_t)BUDGET) best = e;
+    for (int e = 1; e * NP <= NT3; ++e)
+      if (flux_bytes(e, true, staged) <= (size_t)BUDGET && (!staged || e * NP * RB % 16 == 0))
+        best = e;
     return best;
   }
-  static constexpr int EPB3 = pick_epb3();
-  static constexpr int NCOL3 = round_up(NC * EPB3, 8);
+  static_assert(epb3(true) * NP * RB % 16 == 0, "no tile of whole 16-byte pieces");
 
   // ---- face kernel
   // 8-element tiles (the face pass is bound by its gathers' latency: 8.7 ms
@@ -841,32 +839,36 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT),
 // k_volume with the gradients read from HBM (written by the gradient kernel),
 // for the three-kernel pass gradient -> flux-volume -> face.
 //
-// The tile's inputs (NC fields, temperatures, (NC+1) DIM gradients: one
+// STAGED: the tile's inputs (NC fields, temperatures, (NC+1) DIM gradients: one
 // contiguous row of EPB * NP values each) are brought into shared memory by
 // bulk copies (cp.async.bulk), issued as soon as the previous tile's pointwise
 // phase has read its own and running under that tile's divergence; its
 // geometry is computed in the same window into a second buffer.  A node's
 // thread then reads them where the flux needs them: no address arithmetic, no
 // registers held for loads in flight, no wait for DRAM at the start of a tile.
-// Rows that bulk copies cannot move (a row start off 16 bytes: odd NP, an odd
-// number of order-2 float32 elements, an unaligned caller's pointer) are
-// copied by the threads into the same place.  Measured: float64 32^3 p3 2.57 ->
-// 2.46 ms, float32 1260 tetrahedra 23.5 -> 20.2 us; float32 64^3 p3 is the same
-// with and without (7.46 ms: its pointwise arithmetic bounds it).
-template <class R, int DIM, int ORDER, int NS, bool MIX, bool VISC>
+// Measured: float64 32^3 p3 2.57 -> 2.46 ms, float32 1260 tetrahedra 23.5 ->
+// 20.2 us; float32 64^3 p3 is the same with and without (7.46 ms).
+// Not STAGED: rows that bulk copies cannot move (flux_rows_aligned: a row start
+// off 16 bytes, as with an unaligned caller's pointer, an odd number of float32
+// order-2 elements, 2-D float32 orders 1 and 4) are read from global memory by
+// the node's thread.  Right-hand side of the 7-species mixture, float32, threads
+// copying such rows into shared memory -> direct reads: 2-D order 4, 301 x 299
+// cells 1.83 -> 0.99 ms; order 2, 27 x 25 x 25 cells, offset by one value 1.15 ->
+// 0.66 ms.
+template <class R, int DIM, int ORDER, int NS, bool MIX, bool VISC, bool STAGED>
 __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT3), 2)
     k_flux_volume(DGArgs<R> a, GasParams g) {
   using V = VCfg<R, DIM, ORDER, NS, MIX>;
   using S = Simplex<DIM, ORDER>;
   constexpr int NP = V::NP, NF = V::NF, NFP = V::NFP, NFN = V::NFN, NC = V::NC;
-  constexpr int EPB = V::EPB3, MP = V::MP, MT = V::MT, MROW = V::MROW;
-  constexpr int KU = V::KU, KUR = V::KUR, NCOLD = V::NCOL3, NNODE = V::nnode3(V::EPB3);
+  constexpr int EPB = V::epb3(STAGED), MT = V::MT, MROW = V::MROW;
+  constexpr int KU = V::KU, KUR = V::KUR, NCOLD = round_up(NC * EPB, 8), NNODE = V::nnode3(EPB);
   constexpr int FST = V::FST, TW = V::TW, GEO = V::GEO3, DD = DIM * DIM;
   constexpr int AWN = DIM * NP * KU;
   constexpr int ENP = EPB * NP;
-  constexpr int NROW = V::rows3(VISC), RST = round_up(ENP * (int)sizeof(R), 16) / (int)sizeof(R);
+  constexpr int NROW = STAGED ? V::rows3(VISC) : 0, RST = round_up(ENP * (int)sizeof(R), 16) / (int)sizeof(R);
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  R* aw = reinterpret_cast<R*>(smem_raw);                  // [NAC][DIM][MP][KU]
+  R* aw = reinterpret_cast<R*>(smem_raw);                  // [NAC][DIM][NP][KU]
   R* gfl = aw + V::A_FLUX;                                 // [NNODE][FST]
   R* src_s = gfl + NNODE * FST;                            // [NS][ENP]
   R* geo_s = src_s + NS * ENP;                             // [2][EPB][GEO]
@@ -887,29 +889,30 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT3), 2)
     if (MIX && i < V::ROW_G) return i == V::ROW_T ? a.t_op : (own_src ? a.t_src : nullptr);
     return a.grad + (i - V::ROW_G) * EN;
   };
-  const bool bulk = ((reinterpret_cast<uintptr_t>(a.q) | (MIX ? reinterpret_cast<uintptr_t>(a.t_op) : 0) |
-                      (own_src ? reinterpret_cast<uintptr_t>(a.t_src) : 0) |
-                      (VISC ? reinterpret_cast<uintptr_t>(a.grad) : 0)) & 15) == 0 &&
-                    (EN * sizeof(R)) % 16 == 0 && (ENP * sizeof(R)) % 16 == 0;
+  // input *i* of node *gnd*, the tile's node *n*
+  auto value = [&](int i, int n, int64_t gnd) -> R {
+    if constexpr (STAGED)
+      return row_s[i * RST + n];
+    else
+      return row_ptr(i)[gnd];
+  };
   const int ntiles = (a.nowned + EPB - 1) / EPB;
-  // rows of tile *tl*: bulk copies by warp 0 (all threads without them)
+  // rows of tile *tl*: bulk copies by warp 0, what is left of a last tile's rows
+  // (less than 16 bytes each) by all threads
   auto stage_rows = [&](int tl) {
     const int64_t n0 = (int64_t)tl * ENP;
     const int n = imin(ENP, (int)((int64_t)a.nowned * NP - n0));
-    int done_n = 0;
-    if (bulk) {
-      const uint32_t bytes = (uint32_t)(n * sizeof(R)) & ~15u;
-      done_n = bytes / (int)sizeof(R);
-      if (threadIdx.x < 32) {
-        if (threadIdx.x == 0)
-          mbar_expect(&staged, bytes * (uint32_t)(NROW - (MIX && !own_src ? 1 : 0)));
-        __syncwarp();
-        for (int i = threadIdx.x; i < NROW; i += 32) {
-          const R* p = row_ptr(i);
-          if (p && bytes) bulk_load(row_s + i * RST, p + n0, bytes, &staged);
-        }
+    const uint32_t bytes = (uint32_t)(n * sizeof(R)) & ~15u;
+    if (threadIdx.x < 32) {
+      if (threadIdx.x == 0)
+        mbar_expect(&staged, bytes * (uint32_t)(NROW - (MIX && !own_src ? 1 : 0)));
+      __syncwarp();
+      for (int i = threadIdx.x; i < NROW; i += 32) {
+        const R* p = row_ptr(i);
+        if (p && bytes) bulk_load(row_s + i * RST, p + n0, bytes, &staged);
       }
     }
+    const int done_n = bytes / (int)sizeof(R);
     if (done_n < n) {
       const int m = n - done_n;
       for (int i = threadIdx.x; i < NROW * m; i += blockDim.x) {
@@ -951,7 +954,7 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT3), 2)
     }
   };
 
-  if (threadIdx.x == 0) {
+  if (STAGED && threadIdx.x == 0) {
     mbar_init(&staged, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -964,7 +967,7 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT3), 2)
   fill_slots<DIM, ORDER>(slot_s);
   __syncthreads();
   if ((int)blockIdx.x < ntiles) {
-    stage_rows(blockIdx.x);
+    if constexpr (STAGED) stage_rows(blockIdx.x);
     geometry(blockIdx.x, 0, 0, blockDim.x);
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -982,16 +985,19 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT3), 2)
     // the previous tile's divergence has read gfl and src_s; this tile's
     // geometry is complete
     __syncthreads();
-    const bool ok = !bulk || mbar_wait(&staged, it & 1, nullptr);
+    const bool ok = !STAGED || mbar_wait(&staged, it & 1, nullptr);
 
-    for (int n = threadIdx.x; n < ne * NP && ok; n += blockDim.x) {
+    // one node per thread (as a loop: 1 % of the float32 order-3 right-hand side
+    // slower, 2 % of the order-2 one)
+    static_assert(ENP <= V::NT3, "one node per thread");
+    if (const int n = threadIdx.x; n < ne * NP && ok) {
       const int e = n / NP, k = n % NP;
       const int64_t gnd = (int64_t)(e0 + e) * NP + k;
       R qq[NC];
 #pragma unroll
-      for (int c = 0; c < NC; ++c) qq[c] = row_s[c * RST + n];
+      for (int c = 0; c < NC; ++c) qq[c] = value(c, n, gnd);
       NodeState<R, DIM, NS> st;
-      make_state<R, DIM, NS>(qq, MIX ? row_s[V::ROW_T * RST + n] : R(0), g, st);
+      make_state<R, DIM, NS>(qq, MIX ? value(V::ROW_T, n, gnd) : R(0), g, st);
       R fl[NC][DIM];
       inviscid_flux<R, DIM, NS>(st, fl);
 #pragma unroll
@@ -999,14 +1005,13 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT3), 2)
 #pragma unroll
         for (int j = 0; j < DIM; ++j) fl[c][j] = -fl[c][j];
       if constexpr (VISC) {
-        const R* gr = row_s + V::ROW_G * RST + n;
         R gqv[NC][DIM], gt[DIM];
 #pragma unroll
         for (int c = 0; c < NC; ++c)
 #pragma unroll
-          for (int j = 0; j < DIM; ++j) gqv[c][j] = gr[(c * DIM + j) * RST];
+          for (int j = 0; j < DIM; ++j) gqv[c][j] = value(V::ROW_G + c * DIM + j, n, gnd);
 #pragma unroll
-        for (int j = 0; j < DIM; ++j) gt[j] = gr[(NC * DIM + j) * RST];
+        for (int j = 0; j < DIM; ++j) gt[j] = value(V::ROW_G + NC * DIM + j, n, gnd);
         R fv[NC][DIM];
         viscous_flux<R, DIM, NS, MIX>(st, gqv, gt, fv);
 #pragma unroll
@@ -1028,8 +1033,8 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT3), 2)
       if constexpr (MIX && NS > 0) {
         if (sources) {
           R om[NS];
-          production_rates<R, NS>(st.rho, row_s[(own_src ? V::ROW_T + 1 : V::ROW_T) * RST + n],
-                                  st.y, (R)g.zero_level, om);
+          const R ts = STAGED ? row_s[(own_src ? V::ROW_T + 1 : V::ROW_T) * RST + n] : a.t_src[gnd];
+          production_rates<R, NS>(st.rho, ts, st.y, (R)g.zero_level, om);
 #pragma unroll
           for (int sp = 0; sp < NS; ++sp) src_s[sp * ENP + n] = mech<R>().mw[sp] * om[sp];
         }
@@ -1091,12 +1096,16 @@ __global__ void __launch_bounds__((VCfg<R, DIM, ORDER, NS, MIX>::NT3), 2)
       }
     }
     // gfl and the sources are complete, the staged rows have been read
-    if (__syncthreads_or(!ok)) {
-      timeout = true;
-      break;
+    if constexpr (STAGED) {
+      if (__syncthreads_or(!ok)) {
+        timeout = true;
+        break;
+      }
+    } else {
+      __syncthreads();
     }
     if (tile + (int)gridDim.x < ntiles) {
-      stage_rows(tile + gridDim.x);
+      if constexpr (STAGED) stage_rows(tile + gridDim.x);
       // by the last warps, which have the least divergence work
       geometry(tile + gridDim.x, b ^ 1, blockDim.x - 64, 64);
     }

@@ -3,8 +3,9 @@
 * tcgen05 gradients at order 2 (two row blocks of eight elements, rows moved
   in 8-byte pieces), against the mma.sync kernel and the float64 gradients,
   as test_gpu_grad_tc.py does for orders 1 and 3;
-* the flux-volume kernel's staged inputs: rows off 16-byte boundaries are
-  copied by the threads instead of bulk copies, with identical results;
+* the flux-volume kernel's inputs: rows off 16-byte boundaries are read from
+  global memory instead of staged by bulk copies, with identical results; a
+  partition whose last tile's rows end off 16 bytes;
 * the mixture temperature from one polynomial pair per node against the
   species sums (which mechanisms with differing mid temperatures take), with
   iterations that cross the mid temperature.
@@ -67,6 +68,64 @@ def test_flux_rows_off_16_bytes(cuda, dim, order):
         out.append(ns_operator(d, gas, st, {}, species_source_temperature=st.temperature).q)
     assert runtime.read_status(d) == 0
     assert torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("dim,order", [(2, 1), (2, 2), (2, 4), (3, 1), (3, 2), (3, 3)])
+def test_flux_rows_off_16_bytes_float32(cuda, dim, order):
+    """Every input row off 16 bytes, at 4, 8 or 12 bytes of it; the mma.sync
+    gradient kernel on both sides, so that the gradients are the same."""
+    d, od = make_disc("simplex", dim, 4, order, (0.0,) * dim, BOX[:dim], True)
+    assert d.nelements * d.refel.nnodes % 4 == 0
+    cv0, t = reacting_mixture_state([torch.from_numpy(od.nodes[i]) for i in range(dim)], UIUC_7SP,
+                                    seed=2, t_range=(900.0, 1500.0), box=BOX[:dim])
+    gas = _gas()
+    q = cv0.q.to(cuda, torch.float32).contiguous()
+    out = []
+    runtime.set_gradient_kernel("mma_sync")
+    try:
+        for off in (0, 1, 2, 3):
+            buf = torch.empty(q.numel() + 4, dtype=q.dtype, device=cuda)
+            qo = buf[off:off + q.numel()].view(q.shape)
+            qo.copy_(q)
+            assert qo.data_ptr() % 16 == 4 * off
+            st = make_fluid_state(ConservedVars(qo, dim), gas,
+                                  temperature_seed=(t + 3.0).to(cuda, torch.float32))
+            out.append(ns_operator(d, gas, st, {}, species_source_temperature=st.temperature).q)
+    finally:
+        runtime.set_gradient_kernel("auto")
+    assert runtime.read_status(d) == 0
+    for o in out[1:]:
+        assert torch.equal(out[0], o)
+
+
+@pytest.mark.parametrize("order,elems,owned", [(2, 162, 61), (2, 162, 81), (1, 162, 61)])
+def test_last_tile_off_16_bytes_float32(cuda, order, elems, owned):
+    """The first *owned* of *elems* elements through the C entry point, float32:
+    whole rows on 16 bytes, a last tile that ends off them (order 2, odd count),
+    against the same elements of the whole mesh's flux-volume pass."""
+    d, od = make_disc("simplex", 3, 3, order, (0.0,) * 3, BOX, True)
+    assert d.nelements == elems
+    cv0, t = reacting_mixture_state([torch.from_numpy(od.nodes[i]) for i in range(3)], UIUC_7SP,
+                                    seed=2, t_range=(900.0, 1500.0), box=BOX)
+    gas = _gas()
+    st = make_fluid_state(ConservedVars(cv0.q.to(cuda, torch.float32).contiguous(), 3), gas,
+                          temperature_seed=(t + 3.0).to(cuda, torch.float32))
+    dd = runtime.device_discretization(d, cuda)
+    out = []
+    for n in (0, owned):
+        dd.mesh.nowned = n
+        try:
+            rhs = torch.zeros_like(st.cv.q)
+            runtime.ns_rhs(d, st, gas, {}, 0.0, 0, source_temperature=st.temperature, phases=1,
+                           rhs=rhs)
+            gs = runtime._gas_struct(gas, 7, cuda)
+            out.append((rhs[:, :owned].clone(),
+                        runtime.face_records(dd, gs, True, 12)[:owned].clone()))
+        finally:
+            dd.mesh.nowned = 0
+    assert runtime.read_status(d) == 0
+    for a, b in zip(*out):
+        assert torch.equal(a, b)
 
 
 @pytest.mark.parametrize("dtype,tol", [(torch.float64, 1e-12), (torch.float32, 2e-7)])
