@@ -108,10 +108,25 @@ inline int upload_refops_local(int dim, int order, const double* packed64, const
   return MGC_OK;
 }
 
+// per device: the mechanism this unit holds there has one mid temperature
+constexpr int kMechDevices = 64;
+bool g_one_t_mid[kMechDevices] = {};
+
 inline int upload_mechanism_local(const Mechanism* m) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMechDevices) return MGC_E_CUDA;
   if (cudaMemcpyToSymbol(c_mech, m, sizeof(Mechanism)) != cudaSuccess) return MGC_E_CUDA;
   const MechanismT<float> f = narrow_mechanism(*m);
-  return cudaMemcpyToSymbol(c_mech32, &f, sizeof(f)) == cudaSuccess ? MGC_OK : MGC_E_CUDA;
+  if (cudaMemcpyToSymbol(c_mech32, &f, sizeof(f)) != cudaSuccess) return MGC_E_CUDA;
+  g_one_t_mid[dev] = m->one_t_mid != 0;
+  return MGC_OK;
+}
+
+// whether the temperature kernels take the mixture's polynomial pair
+// (MixturePoly) on the current device
+inline bool one_t_mid_here() {
+  int dev = 0;
+  return cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMechDevices && g_one_t_mid[dev];
 }
 
 // What the runtime has answered before for a kernel on a device: the largest
@@ -436,7 +451,8 @@ inline int mixture_state_mixed_dim(int ns, int64_t nnodes, const float* q, const
   const int nt = 256;
   // grid-stride loop: one wave of resident blocks, so that no second,
   // partly filled wave runs at a fraction of the machine
-  auto kern = k_mixture_state_mixed<DIM, 7>;
+  auto kern = one_t_mid_here() ? k_mixture_state_mixed<DIM, 7, true>
+                               : k_mixture_state_mixed<DIM, 7, false>;
   int nb = 0;
   const int rc = persistent_grid(kern, nt, 0, (nnodes + nt - 1) / nt, &nb);
   if (rc) return rc;
@@ -449,7 +465,8 @@ inline int mixture_state_dim(int ns, int64_t nnodes, const R* q, const R* tseed,
                              int32_t* status, const GasParams& g, cudaStream_t s) {
   if (ns != 7) return MGC_E_UNSUPPORTED;
   const int nt = 256;
-  auto kern = k_mixture_state<R, DIM, 7>;   // grid-stride: one wave of resident blocks
+  // grid-stride: one wave of resident blocks
+  auto kern = one_t_mid_here() ? k_mixture_state<R, DIM, 7, true> : k_mixture_state<R, DIM, 7, false>;
   int nb = 0;
   const int rc = persistent_grid(kern, nt, 0, (nnodes + nt - 1) / nt, &nb);
   if (rc) return rc;

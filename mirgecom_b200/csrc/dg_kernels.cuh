@@ -377,11 +377,12 @@ __device__ __noinline__ void mengaldo_grad_value(const DGArgs<R> a, const GasPar
 // more than 1e-6 of T1, or whose temperature is not positive and finite,
 // sets ST_NEWTON_MISS in *status*.  The temperatures written are the
 // reference's either way.
-template <class R, int DIM, int NS>
+template <class R, int DIM, int NS, bool POLY>
 __global__ void __launch_bounds__(256) k_mixture_state(int64_t nnodes, const R* __restrict__ q,
                                                        const R* __restrict__ tseed,
                                                        R* __restrict__ t1, R* __restrict__ t2,
                                                        int32_t* status, GasParams g) {
+  constexpr int FORM = POLY ? NEWTON_POLY : NEWTON_SUMS;
   constexpr int NC = DIM + 2 + NS;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   bool miss = false;
@@ -389,16 +390,16 @@ __global__ void __launch_bounds__(256) k_mixture_state(int64_t nnodes, const R* 
     R qq[NC];
 #pragma unroll
     for (int c = 0; c < NC; ++c) qq[c] = q[(int64_t)c * nnodes + n];
-    const R ta = node_temperature<R, DIM, NS>(qq, tseed[n], g);
+    const R ta = node_temperature<R, DIM, NS, FORM>(qq, tseed[n], g);
     t1[n] = ta;
     R tb;
     if (t2) {
-      tb = node_temperature<R, DIM, NS>(qq, ta, g);
+      tb = node_temperature<R, DIM, NS, FORM>(qq, ta, g);
       t2[n] = tb;
     } else {
       GasParams g1 = g;
       g1.niter = 1;
-      tb = node_temperature<R, DIM, NS>(qq, ta, g1);
+      tb = node_temperature<R, DIM, NS, FORM>(qq, ta, g1);
     }
     miss |= !(ta > R(0) && tb > R(0) && fabs(tb - ta) <= R(1e-6) * ta && ta < R(1e30));
   }
@@ -415,7 +416,7 @@ __global__ void __launch_bounds__(256) k_mixture_state(int64_t nnodes, const R* 
 // rejected result is recomputed from the plain guess (seed).  iters
 // (optional) receives the float32 iteration count per node, with 1000
 // added when the fallback ran; ST_NEWTON_MISS flags nodes that fail both.
-template <int DIM, int NS>
+template <int DIM, int NS, bool POLY>
 __global__ void __launch_bounds__(256) k_mixture_state_mixed(
     int64_t nnodes, const float* __restrict__ q, const float* __restrict__ tseed,
     const float* __restrict__ tguess, float* __restrict__ tout, int32_t* __restrict__ iters,
@@ -427,9 +428,9 @@ __global__ void __launch_bounds__(256) k_mixture_state_mixed(
     float qq[NC];
 #pragma unroll
     for (int c = 0; c < NC; ++c) qq[c] = q[(int64_t)c * nnodes + n];
-    MixedEnergy<NS> en;
+    MixedEnergy<NS, POLY> en;
     double e64;
-    mixed_newton_inputs<DIM, NS>(qq, en.yw, e64);
+    mixed_newton_inputs<DIM>(qq, en, e64);
     const float e32 = (float)e64;
     en.start(tguess ? tguess[n] : tseed[n]);
     int used = 0;
@@ -438,7 +439,7 @@ __global__ void __launch_bounds__(256) k_mixture_state_mixed(
     // attempt 0: learned guess (when given); attempt 1: the plain guess (seed)
     for (int attempt = tguess ? 0 : 1; attempt < 2 && !ok; ++attempt) {
       t = (attempt == 0) ? tguess[n] : tseed[n];
-      ok = mixed_newton<NS>(en, e32, e64, t, maxit, (double)rtol, used);
+      ok = mixed_newton(en, e32, e64, t, maxit, (double)rtol, used);
       if (!ok && attempt == 0) used += 1000;
     }
     if (!ok) miss = true;

@@ -643,7 +643,7 @@ constexpr float kWarmSeedK = 4.0f;
 // shared memory, and each lane solves its node's temperature with
 // mixed_newton from the guess, falling back to the seed when the float64
 // residual check fails (iteration count + 1000 marks it).
-template <int DIM, int NS>
+template <int DIM, int NS, bool POLY>
 __global__ void __launch_bounds__(WARPS * 32, 6) k_mixture_state_learned(
     int64_t n, const float* __restrict__ q, const float* __restrict__ tseed, Net net,
     float* __restrict__ tout, int32_t* __restrict__ iters, int maxit, double rtol,
@@ -669,9 +669,9 @@ __global__ void __launch_bounds__(WARPS * 32, 6) k_mixture_state_learned(
     float qq[NC];
 #pragma unroll
     for (int c = 0; c < NC; ++c) qq[c] = valid ? q[(int64_t)c * n + s] : (c == 0 ? 1.f : 0.f);
-    MixedEnergy<NS> en;
+    MixedEnergy<NS, POLY> en;
     double e64;
-    mixed_newton_inputs<DIM, NS>(qq, en.yw, e64);
+    mixed_newton_inputs<DIM>(qq, en, e64);
     const float e32 = (float)e64;
     // one float32 step from the seed; a warm warp continues from there
     const float ts = valid ? tseed[s] : 1000.f;
@@ -690,7 +690,7 @@ __global__ void __launch_bounds__(WARPS * 32, 6) k_mixture_state_learned(
       float f[8];
       f[0] = e32;
 #pragma unroll
-      for (int k = 0; k < 7; ++k) f[1 + k] = k < NS ? (float)(en.yw[k] * mech<double>().mw[k]) : 0.f;
+      for (int k = 0; k < 7; ++k) f[1 + k] = k < NS ? en.y(k) : 0.f;
 #pragma unroll
       for (int j = 0; j < KIN; j += 2) {
         const float v0 = j < 8 ? (f[j] - net.in_shift[j]) * net.in_scale[j] : 0.f;
@@ -717,15 +717,15 @@ __global__ void __launch_bounds__(WARPS * 32, 6) k_mixture_state_learned(
       // so that none of them stays live across the network
 #pragma unroll
       for (int c = 0; c < NC; ++c) qq[c] = valid ? q[(int64_t)c * n + s] : (c == 0 ? 1.f : 0.f);
-      mixed_newton_inputs<DIM, NS>(qq, en.yw, e64);
+      mixed_newton_inputs<DIM>(qq, en, e64);
       en.start(t);
     }
     if (valid) {
-      bool ok = mixed_newton<NS>(en, e32, e64, t, mx, rtol, used);
+      bool ok = mixed_newton(en, e32, e64, t, mx, rtol, used);
       if (!ok) {
         used += 1000;
         t = ts;
-        ok = mixed_newton<NS>(en, e32, e64, t, maxit, rtol, used);
+        ok = mixed_newton(en, e32, e64, t, maxit, rtol, used);
       }
       if (!ok) miss = true;
       tout[s] = t;
@@ -738,6 +738,7 @@ __global__ void __launch_bounds__(WARPS * 32, 6) k_mixture_state_learned(
 // }}}
 
 bool g_mech_ready_mlp[64] = {};
+bool g_one_t_mid_mlp[64] = {};
 
 }  // namespace
 
@@ -750,6 +751,7 @@ int mlp_upload_mechanism(const Mechanism* m) {
   if (cudaMemcpyToSymbol(c_mech, m, sizeof(Mechanism)) != cudaSuccess) return MGC_E_CUDA;
   const MechanismT<float> f = narrow_mechanism(*m);
   if (cudaMemcpyToSymbol(c_mech32, &f, sizeof(f)) != cudaSuccess) return MGC_E_CUDA;
+  g_one_t_mid_mlp[dev] = m->one_t_mid != 0;
   g_mech_ready_mlp[dev] = true;
   return MGC_OK;
 }
@@ -838,7 +840,9 @@ int mgc_mixture_temperature_learned_f32(int dim, const mgc_gas_t* gas, int64_t n
   if (!g_mech_ready_mlp[dev]) return MGC_E_NOT_READY;
   const Net net = make_net(mlp);
   cudaStream_t s = (cudaStream_t)stream;
-  auto kern = dim == 3 ? k_mixture_state_learned<3, 7> : k_mixture_state_learned<2, 7>;
+  const bool poly = g_one_t_mid_mlp[dev];
+  auto kern = dim == 3 ? (poly ? k_mixture_state_learned<3, 7, true> : k_mixture_state_learned<3, 7, false>)
+                       : (poly ? k_mixture_state_learned<2, 7, true> : k_mixture_state_learned<2, 7, false>);
   // grid-stride over 32-node chunks: one wave of resident blocks
   int sms = 0, per_sm = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||

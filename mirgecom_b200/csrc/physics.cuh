@@ -191,26 +191,20 @@ __device__ __forceinline__ R species_s_r(int s, const TPow<R>& p, R logt) {
 }
 
 // mixture e (J/kg) and c_v (J/kg/K) at temperature t
-template <class R, int NS, class Y>
-__device__ __forceinline__ void mixture_e_cv_yw(const Y* yw, R t, R& e, R& cv) {
+template <class R, int NS>
+__device__ __forceinline__ void mixture_e_cv(const R* y, R t, R& e, R& cv) {
   const TPow<R> p(t);
   R se = 0, scv = 0;
 #pragma unroll
   for (int s = 0; s < NS; ++s) {
     R cps, hs;
     nasa_cp_h<R>(s, p, cps, hs);
-    se += (R)yw[s] * (hs - (R)1);
-    scv += (R)yw[s] * (cps - (R)1);
+    const R yw = y[s] * mech<R>().inv_mw[s];
+    se += yw * (hs - (R)1);
+    scv += yw * (cps - (R)1);
   }
   e = (R)kGasConstant * t * se;
   cv = (R)kGasConstant * scv;
-}
-template <class R, int NS>
-__device__ __forceinline__ void mixture_e_cv(const R* y, R t, R& e, R& cv) {
-  R yw[NS];
-#pragma unroll
-  for (int s = 0; s < NS; ++s) yw[s] = y[s] * mech<R>().inv_mw[s];
-  mixture_e_cv_yw<R, NS>(yw, t, e, cv);
 }
 
 // e(T) and c_v(T) of a mixture as ONE polynomial pair: with every species in
@@ -218,8 +212,10 @@ __device__ __forceinline__ void mixture_e_cv(const R* y, R t, R& e, R& cv) {
 // sum_k (Y_k / W_k) a_kj, formed once per node (6 NS multiply-adds); a Newton
 // step then takes 10 instead of ~25 NS (mixture_e_cv).  *hi* is the range the
 // coefficients hold; a step that crosses t_mid forms them again.  Mechanisms
-// whose species differ in t_mid (one_t_mid false) use mixture_e_cv.  (The
-// species sums were bound by their constant loads, one per multiply-add.)
+// whose species differ in t_mid (one_t_mid false) use mixture_e_cv, in kernels
+// of their own: chosen in the kernel, the two forms share its registers (the
+// species sums of 2^20 cold nodes with the learned guess 148 -> 188 us).  (The
+// species sums are bound by their constant loads, one per multiply-add.)
 // Temperature kernels of the 7-species mixture, CUDA events: float64 32^3 p3
 // 622 -> 269 us, float32 40^3 p2 157 -> 130 us, with the learned guess and warm
 // seeds 64^3 p3 1.41 -> 0.82 ms.
@@ -317,22 +313,23 @@ __device__ __forceinline__ R conc_pow(R c, R o) {
 
 // T_{i+1} = T_i + (e - e(T_i)) / c_v(T_i), fixed count
 template <class R, int NS>
-__device__ __forceinline__ R newton_temperature(R e, R tguess, const R* y, int niter) {
-  R t = tguess;
-  if (mech<R>().one_t_mid) {
-    R yw[NS];
+__device__ __forceinline__ R newton_poly(R e, R tguess, const R* y, int niter) {
+  R t = tguess, yw[NS];
 #pragma unroll
-    for (int k = 0; k < NS; ++k) yw[k] = y[k] * mech<R>().inv_mw[k];
-    MixturePoly<R> p;
-    p.template form<NS>(yw, t);
-    for (int it = 0; it < niter; ++it) {
-      if (!p.holds(t)) p.template form<NS>(yw, t);
-      R em, cv;
-      p.eval(t, em, cv);
-      t = t + (e - em) / cv;
-    }
-    return t;
+  for (int k = 0; k < NS; ++k) yw[k] = y[k] * mech<R>().inv_mw[k];
+  MixturePoly<R> p;
+  p.template form<NS>(yw, t);
+  for (int it = 0; it < niter; ++it) {
+    if (!p.holds(t)) p.template form<NS>(yw, t);
+    R em, cv;
+    p.eval(t, em, cv);
+    t = t + (e - em) / cv;
   }
+  return t;
+}
+template <class R, int NS>
+__device__ __forceinline__ R newton_sums(R e, R tguess, const R* y, int niter) {
+  R t = tguess;
   for (int it = 0; it < niter; ++it) {
     R em, cv;
     mixture_e_cv<R, NS>(y, t, em, cv);
@@ -340,31 +337,31 @@ __device__ __forceinline__ R newton_temperature(R e, R tguess, const R* y, int n
   }
   return t;
 }
-
-// Newton inputs of the mixed form from a float32 conserved state: the specific
-// internal energy and Y_k / W_k in float64 (one reciprocal of rho).
-template <int DIM, int NS>
-__device__ __forceinline__ void mixed_newton_inputs(const float* qq, double* yw, double& e64) {
-  const double irho = 1.0 / (double)qq[0];
-#pragma unroll
-  for (int k = 0; k < NS; ++k)
-    yw[k] = ((double)qq[2 + DIM + k] * irho) * mech<double>().inv_mw[k];
-  double ked = 0;
-#pragma unroll
-  for (int i = 0; i < DIM; ++i) ked += (double)qq[2 + i] * (double)qq[2 + i];
-  e64 = ((double)qq[1] - 0.5 * ked * irho) * irho;
+// which form a kernel is compiled for (NEWTON_ANY: both, the mechanism's
+// one_t_mid read there)
+enum NewtonForm { NEWTON_ANY = 0, NEWTON_POLY = 1, NEWTON_SUMS = 2 };
+template <class R, int NS, int FORM>
+__device__ __forceinline__ R newton_temperature(R e, R tguess, const R* y, int niter) {
+  if (FORM == NEWTON_POLY || (FORM == NEWTON_ANY && mech<R>().one_t_mid))
+    return newton_poly<R, NS>(e, tguess, y, niter);
+  return newton_sums<R, NS>(e, tguess, y, niter);
 }
 
-// The Newton's e(T), c_v(T) of one node of the mixed form: the polynomial
-// pair formed once in float64 and its float32 rounding (one_t_mid), or the
-// species sums.
+// The Newton's e(T), c_v(T) of one node of the mixed form.  POLY (one_t_mid): the
+// polynomial pair formed once in float64 and its float32 rounding; otherwise
+// the species sums of float64 and float32 mass fractions.
+template <int NS, bool POLY> struct MixedEnergy;
+
 template <int NS>
-struct MixedEnergy {
+struct MixedEnergy<NS, true> {
   MixturePoly<double> p;
   float c[5], b[5], a5;      // float32: c_v and e coefficients, / R
   double yw[NS];             // Y_k / W_k
 
-  __device__ __forceinline__ void form(float t) {
+  __device__ __forceinline__ void set(int k, double y) { yw[k] = y * mech<double>().inv_mw[k]; }
+  __device__ __forceinline__ float y(int k) const { return (float)(yw[k] * mech<double>().mw[k]); }
+  // form the pair of the range that holds t
+  __device__ __forceinline__ void start(float t) {
     p.template form<NS>(yw, (double)t);
 #pragma unroll
     for (int j = 0; j < 5; ++j) c[j] = (float)p.c[j];
@@ -375,24 +372,50 @@ struct MixedEnergy {
     b[4] = c[4] * 0.2f;
     a5 = (float)p.a5;
   }
-  __device__ __forceinline__ void start(float t) {
-    if (mech<float>().one_t_mid) form(t);
-  }
-  __device__ __forceinline__ void ready(float t) {
-    if (mech<float>().one_t_mid && !p.holds((double)t)) form(t);
-  }
   __device__ __forceinline__ void eval(float t, float& e, float& cv) {
-    if (!mech<float>().one_t_mid) return mixture_e_cv_yw<float, NS>(yw, t, e, cv);
-    ready(t);
+    if (!p.holds((double)t)) start(t);
     e = (float)kGasConstant * (t * (b[0] + t * (b[1] + t * (b[2] + t * (b[3] + t * b[4])))) + a5);
     cv = (float)kGasConstant * (c[0] + t * (c[1] + t * (c[2] + t * (c[3] + t * c[4]))));
   }
   __device__ __forceinline__ void eval(double t, double& e, double& cv) {
-    if (!mech<float>().one_t_mid) return mixture_e_cv_yw<double, NS>(yw, t, e, cv);
-    ready((float)t);
+    if (!p.holds((double)(float)t)) start((float)t);
     p.eval(t, e, cv);
   }
 };
+
+template <int NS>
+struct MixedEnergy<NS, false> {
+  float yf[NS];
+  double yd[NS];
+
+  __device__ __forceinline__ void set(int k, double y) {
+    yd[k] = y;
+    yf[k] = (float)y;
+  }
+  __device__ __forceinline__ float y(int k) const { return yf[k]; }
+  __device__ __forceinline__ void start(float) {}
+  __device__ __forceinline__ void eval(float t, float& e, float& cv) const {
+    mixture_e_cv<float, NS>(yf, t, e, cv);
+  }
+  __device__ __forceinline__ void eval(double t, double& e, double& cv) const {
+    mixture_e_cv<double, NS>(yd, t, e, cv);
+  }
+};
+
+// Newton inputs of the mixed form from a float32 conserved state: the specific
+// internal energy (*e64*) and the mass fractions in float64 (one reciprocal of
+// rho).
+template <int DIM, int NS, bool POLY>
+__device__ __forceinline__ void mixed_newton_inputs(const float* qq, MixedEnergy<NS, POLY>& en,
+                                                    double& e64) {
+  const double irho = 1.0 / (double)qq[0];
+#pragma unroll
+  for (int k = 0; k < NS; ++k) en.set(k, (double)qq[2 + DIM + k] * irho);
+  double ked = 0;
+#pragma unroll
+  for (int i = 0; i < DIM; ++i) ked += (double)qq[2 + i] * (double)qq[2 + i];
+  e64 = ((double)qq[1] - 0.5 * ked * irho) * irho;
+}
 
 // Mixed-precision temperature solve of one node from the start value *t*.
 // Newton converges quadratically: after a step dT the remaining error is
@@ -403,8 +426,8 @@ struct MixedEnergy {
 // rtol |T| (the relative temperature-update tolerance the reference drivers
 // check: mirgecom examples/autoignition.py:526-530).  Returns acceptance;
 // *used* counts float32 iterations.
-template <int NS>
-__device__ __forceinline__ bool mixed_newton(MixedEnergy<NS>& en, float e32, double e64, float& t,
+template <int NS, bool POLY>
+__device__ __forceinline__ bool mixed_newton(MixedEnergy<NS, POLY>& en, float e32, double e64, float& t,
                                              int maxit, double rtol, int& used) {
   const float k = mech<float>().newton_k;
   const float rt = (float)rtol;
@@ -583,7 +606,7 @@ __device__ __forceinline__ void make_state_light(const R* q, R p, R c, R gamma,
 }
 
 // Temperature of a node from q (ideal: closed form; mixture: Newton from seed)
-template <class R, int DIM, int NS>
+template <class R, int DIM, int NS, int FORM = NEWTON_ANY>
 __device__ __forceinline__ R node_temperature(const R* q, R seed, const GasParams& g) {
   R ke = 0;
 #pragma unroll
@@ -598,7 +621,7 @@ __device__ __forceinline__ R node_temperature(const R* q, R seed, const GasParam
 #pragma unroll
     for (int k = 0; k < NS; ++k) y[k] = q[2 + DIM + k] / q[0];
     const R e = (q[1] - ke) / q[0];
-    return newton_temperature<R, NS>(e, seed, y, g.niter);
+    return newton_temperature<R, NS, FORM>(e, seed, y, g.niter);
   }
   return seed;
 }

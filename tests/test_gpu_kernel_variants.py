@@ -149,3 +149,34 @@ def test_temperature_polynomial_against_species_sums(cuda, dtype, tol):
                               temperature_seed=seed.to(cuda, dtype))
         res.append(st.temperature.double().cpu().numpy())
     assert np.max(np.abs(res[0] - res[1]) / res[1]) < tol
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("cold", [False, True])
+def test_learned_temperature_of_both_mechanism_forms(cuda, dim, cold):
+    """The learned-guess kernel of a mechanism with one mid temperature (the
+    polynomial pair) and of one without (species sums), warm warps and warps
+    that run the network, a ragged last warp: 2e-7 of each other, two float32
+    roundings of T (6e-8 each) and two accepted residuals (1e-8)."""
+    from mirgecom_b200.learned_guess import TemperatureMLP
+    g = torch.Generator().manual_seed(4)
+    n = 4099
+    x = [torch.rand(n, generator=g, dtype=torch.float64) * b for b in BOX[:dim]]
+    cv0, t = reacting_mixture_state(x, UIUC_7SP, seed=3, box=BOX[:dim])
+    other = copy.deepcopy(UIUC_7SP)
+    other.t_mid = UIUC_7SP.t_mid.copy()
+    other.t_mid[-1] += 1e-9
+    net = TemperatureMLP(cuda, seed=0)
+    e, y, tt = TemperatureMLP.training_pairs(UIUC_7SP, 1 << 13, cuda, seed=0)
+    net.fit(e, y, tt, steps=100, batch=1 << 13, lr=3e-3, seed=0)
+    res = []
+    for mech in (UIUC_7SP, other):
+        gas = GasModel(eos=PyrometheusMixture(mech, temperature_niter=12, learned_guess=net))
+        st = make_fluid_state(ConservedVars(cv0.q.to(cuda, torch.float32).contiguous(), dim), gas,
+                              temperature_seed=300.0 if cold else (t + 2.0).to(cuda, torch.float32))
+        res.append(st.temperature.double().cpu().numpy())
+    assert int(runtime.state_status_word(cuda).item()) == 0
+    assert np.max(np.abs(res[0] - res[1]) / res[1]) < 2e-7
+    # and of the temperatures the state was made from, to the float32 state's
+    # roundings of the energy (formation enthalpies of ~1e7 J/kg over c_v T)
+    assert np.max(np.abs(res[0] - t.numpy()) / t.numpy()) < 1e-4
