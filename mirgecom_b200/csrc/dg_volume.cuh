@@ -148,9 +148,10 @@ struct VCfg {
   // whole rounds (order-3 tetrahedra: 320 in two; with 128 the third round is
   // half empty, 64^3 float32 3.27 -> 3.10 ms); 128 elsewhere (order 2 in one
   // round of 192: 0.50 -> 0.62 ms at 40^3, four blocks hide less latency than
-  // six)
+  // six).  The four fields of the 2-D ideal gas fit seven blocks (72 registers:
+  // unbounded, order 1 takes 74 and six blocks, 600 x 600 cells 0.90 -> 0.85 ms)
   static constexpr int NT2 = TF32 && (8 * NFN) % 160 == 0 ? 160 : 128;
-  static constexpr int MINB2 = TF32 ? 800 / NT2 : 4;
+  static constexpr int MINB2 = TF32 ? (NC == 4 ? 7 : 800 / NT2) : 4;
   static constexpr int KFR = round_up(NFN, KSTEP);
   static constexpr int KF = Tile<R>::stride(KFR);
   static constexpr int A_FACE = NAC * MP * KF;
