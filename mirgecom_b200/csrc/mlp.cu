@@ -805,11 +805,15 @@ int mgc_mlp_train_grad(int64_t n, const float* x, const float* target, const mgc
   if (cudaMemsetAsync(loss, 0, sizeof(float), s) != cudaSuccess) return MGC_E_CUDA;
   const Net net = make_net(w);
   // resident blocks only: each stages the weights once for its tiles
-  const int nb = imin_(grid_for((n + 15) / 16), 148 * kTrainBlocks);
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return MGC_E_CUDA;
+  const int nb = imin_(grid_for((n + 15) / 16), sms * kTrainBlocks);
   k_mlp_fwd_bwd<<<nb, WARPS * 32, 0, s>>>(n, x, target, net, xb, h1b, dz1b, dz2b, grad, loss,
                                          1.0f / (float)n);
   const int64_t nch = (n + CH - 1) / CH;
-  const int nbw = (int)(nch < 148 * 2 ? nch : 148 * 2);
+  const int nbw = (int)(nch < sms * 2 ? nch : sms * 2);
   k_mlp_wgrad<<<nbw, WARPS * 32, 0, s>>>(n, dz2b, h1b, dz1b, xb, grad + P_W2, grad + P_W1);
   return cudaGetLastError() == cudaSuccess ? MGC_OK : MGC_E_CUDA;
 }
