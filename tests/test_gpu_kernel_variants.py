@@ -17,9 +17,9 @@ import numpy as np
 import pytest
 import torch
 
-from cases import make_disc
+from cases import assert_fields_close, inviscid_flux_floor, make_disc, perturbed_state_np
 from mirgecom_b200 import runtime
-from mirgecom_b200.eos import PyrometheusMixture
+from mirgecom_b200.eos import IdealSingleGas, PyrometheusMixture
 from mirgecom_b200.fluid import ConservedVars
 from mirgecom_b200.gas_model import GasModel, make_fluid_state
 from mirgecom_b200.initializers import reacting_mixture_state
@@ -96,6 +96,28 @@ def test_flux_rows_off_16_bytes_float32(cuda, dim, order):
     assert runtime.read_status(d) == 0
     for o in out[1:]:
         assert torch.equal(out[0], o)
+
+
+@pytest.mark.parametrize("order", [1, 4])
+def test_flux_rows_of_odd_2d_meshes_float32(cuda, order):
+    """Rows whose pitch is off 16 bytes (an odd number of cells of odd-sized
+    elements), against the float64 right-hand side at the mixed form's bar."""
+    d, od = make_disc("simplex", 2, 5, order, (0.0,) * 2, (1.0, 0.7), True)
+    assert d.nelements * d.refel.nnodes * 4 % 16 != 0
+    q = perturbed_state_np(od.nodes, 2, 0, seed=order)
+    gas = GasModel(eos=IdealSingleGas(),
+                   transport=SimpleTransport(viscosity=2e-2, thermal_conductivity=3e-2))
+    saved, out = runtime.RHS_PATH, []
+    runtime.RHS_PATH = "gradient_volume_face"
+    try:
+        for dtype in (torch.float32, torch.float64):
+            cv = ConservedVars(torch.from_numpy(q).to(cuda, dtype), 2)
+            out.append(ns_operator(d, gas, make_fluid_state(cv, gas), {}).q)
+    finally:
+        runtime.RHS_PATH = saved
+    assert runtime.read_status(d) == 0
+    floor = inviscid_flux_floor(q, 2, 0.7 / 5 / order ** 2)
+    assert_fields_close(out[0].double().cpu().numpy(), out[1].cpu().numpy(), 5e-5, floor=floor)
 
 
 @pytest.mark.parametrize("order,elems,owned", [(2, 162, 61), (2, 162, 81), (1, 162, 61)])
