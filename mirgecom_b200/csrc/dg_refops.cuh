@@ -17,11 +17,11 @@
 //
 // The matrices W and LIFT live in a global-memory table: every kernel reads
 // them once per CTA, one entry per thread, to build its tensor-core operands
-// in shared memory.  (From constant memory those per-lane addresses replay one
-// by one; one call of the reacting p3 right-hand side on 1260 tetrahedra,
-// float32: 90.6 us from constant memory, 86.1 us from the table, the 24^3 p3
-// Taylor-Green one in float64 830 and 824 us.)  NREF and FSR, a few values
-// each thread reads for its face, stay in constant memory.
+// in shared memory: from constant memory those per-lane addresses replay one by
+// one.  (The whole call shows it little: 24^3 p3 Taylor-Green, float64, 830 us
+// from constant memory, 824 us from the table; 1260 reacting tetrahedra inside
+// the noise of the host path.)  NREF and FSR, a few values each thread reads for
+// its face, stay in constant memory.
 #pragma once
 #include <cstdint>
 

@@ -23,9 +23,9 @@
 // Against gradient, node-flux and surface kernels (18 gradient values per node
 // written and read, 20 flux values written and read per node) the two kernels
 // move about 320 bytes per node instead of 800.  48^3 order-4 Taylor-Green
-// right-hand side: 6.27 -> 2.83 ms (volume 2.00: shared-memory reads, 57 % of
-// the L1 data peak, and FP64; face 0.82: latency of the gathers); 990 order-2
-// elements 30.5 -> 15.1 us on the device.
+// right-hand side: 6.27 -> 2.83 ms (volume 2.01: shared-memory reads, 59 % of
+// the L1 data peak, and latency at 18 % of the warps; face 0.83: latency of the
+// gathers); 990 order-2 elements 30.5 -> 15.2 us on the device.
 #pragma once
 #include "hex_kernels.cuh"
 

@@ -217,8 +217,8 @@ __device__ __forceinline__ void mixture_e_cv(const R* y, R t, R& e, R& cv) {
 // species sums of 2^20 cold nodes with the learned guess 148 -> 188 us).  (The
 // species sums are bound by their constant loads, one per multiply-add.)
 // Temperature kernels of the 7-species mixture, CUDA events: float64 32^3 p3
-// 622 -> 269 us, float32 40^3 p2 157 -> 130 us, with the learned guess and warm
-// seeds 64^3 p3 1.41 -> 0.82 ms.
+// 622 -> 265 us, float32 40^3 p2 157 -> 96 us, with the learned guess and warm
+// seeds 64^3 p3 1.41 -> 0.70 ms (0.82 with both forms in one kernel).
 template <class R>
 struct MixturePoly {
   R c[5];      // c_v / R = c0 + c1 t + .. + c4 t^4
@@ -300,8 +300,8 @@ __device__ __forceinline__ R conc_pow(R c, R o) {
   if constexpr (sizeof(R) == 4) {
     return c > 0.f ? expf(o * logf(c)) : 0.f;
   } else {
-    // the orders of the usual global mechanisms, an order of magnitude
-    // cheaper than pow (every lane takes the same branch)
+    // orders 1/2 and 3/4, an order of magnitude cheaper than pow, which the
+    // other orders keep (every lane takes the same branch)
     if (o == R(0.5)) return sqrt(c);
     if (o == R(0.75)) {
       const R s = sqrt(c);

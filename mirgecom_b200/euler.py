@@ -3,11 +3,13 @@
 ``euler_operator`` keeps the reference signature.  The RHS
 ``-div_operator(F_I, F*_I)`` -- volume flux, trace pairs, numerical flux,
 boundary fluxes, weak divergence, face lift and inverse mass -- runs on the
-device (``runtime.euler_rhs``): on simplicial meshes two kernels through
-``mgc_operator`` (a volume kernel for the pointwise fluxes, face-node records
-and the volume part of the divergence, a face kernel for the numerical
-fluxes and the lift); on hexahedra two kernels of the same kind through
-``mgc_rhs_hex`` in float64, the split divergence pass in float32.
+device (``runtime.euler_rhs``).  On simplicial meshes by default: mixtures,
+walls and partitions in two kernels through ``mgc_operator`` (a volume kernel for
+the pointwise fluxes, face-node records and the volume part of the divergence, a
+face kernel for the numerical fluxes and the lift), the ideal gas without walls
+in the split divergence pass (node flux records, then surface and lift).  On
+hexahedra two kernels through ``mgc_rhs_hex`` in float64, the split divergence
+pass in float32.
 """
 
 from __future__ import annotations

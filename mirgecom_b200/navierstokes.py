@@ -1,16 +1,18 @@
 """Navier-Stokes operator, mirroring mirgecom/navierstokes.py:129-575.
 
 ``ns_operator`` keeps the reference signature and computes
-div(F_V - F_I) with BR1 gradients on the device (``runtime.ns_rhs``): on
-simplicial meshes in two kernels through ``mgc_operator`` (a volume kernel
-that keeps the gradients on chip and evaluates the pointwise fluxes and the
-volume part of the divergence, and a face kernel for the numerical fluxes and
-the lift); on hexahedra as the same two kernels through ``mgc_rhs_hex`` in
-float64, as a gradient pass and a split divergence pass in float32 or where the
-gradients are asked for.
+div(F_V - F_I) with BR1 gradients on the device (``runtime.ns_rhs``).  On
+simplicial meshes by default: mixtures, walls and partitions through
+``mgc_operator`` in three kernels (gradients, then the pointwise fluxes with the
+volume part of the divergence, then the numerical fluxes and the lift), the
+ideal gas without walls as a gradient pass and a split divergence pass
+(``runtime.RHS_PATH`` lists the other layouts).  On hexahedra through
+``mgc_rhs_hex`` in float64 (a volume kernel that keeps the gradients on chip and
+a face kernel), as a gradient pass and a split divergence pass in float32 or
+where the gradients are asked for.
 For a reacting mixture the species source terms (the driver-side
 ``eos.get_species_source_terms`` of examples/gas-in-box.py:702-705) are
-fused into the volume kernel by passing ``species_source_temperature``.
+fused into the flux kernel by passing ``species_source_temperature``.
 """
 
 from __future__ import annotations

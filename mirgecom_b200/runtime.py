@@ -295,9 +295,13 @@ def _operator_temperature(state):
 #   "fused"        two kernels: gradients, fused divergence -- mgc_ns_grad* +
 #                  mgc_ns_rhs* (mgc_euler_rhs* for the Euler operator)
 #   "auto"         "gradient_volume_face" for mixtures, Mengaldo boundaries and
-#                  kernel phases (partitions); "split" otherwise (the ideal gas
-#                  without walls: 0.55 ms against 0.585 ms for the 24^3 p3
-#                  Taylor-Green right-hand side)
+#                  kernel phases (partitions); "split" otherwise: the ideal gas
+#                  without walls.  Taylor-Green right-hand side, order 3, float64,
+#                  split / volume_face / gradient_volume_face on the device: 5^3
+#                  cells 48 / 46 / 52 us, 10^3 81 / 84 / 87 us, 24^3 0.69 / 0.77 /
+#                  0.74 ms, 48^3 5.1 / 5.8 / 5.5 ms; float32: 5^3 48 / 38 / 48 us,
+#                  10^3 69 / 63 / 67 us, 24^3 0.44 / 0.47 / 0.44 ms, 48^3 3.1 / 3.4 /
+#                  3.1 ms
 # Tensor-product hexahedra take mgc_rhs_hex in float64 (two kernels, gradients
 # on chip) unless the caller wants the gradients, and "split" otherwise.
 RHS_PATH = "auto"
