@@ -23,6 +23,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 
 #include "physics.cuh"
@@ -627,6 +628,19 @@ int grid_for(int64_t tiles) {
   return nb < 1 ? 1 : (int)nb;
 }
 
+// multiprocessors of the current device, asked once per device (0: failed)
+int sm_count() {
+  static std::atomic<int> known[64];
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  n = known[dev].load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    known[dev].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
 // {{{ mixture temperature with the learned guess (fused)
 
 // A seed whose first Newton step is at most this large already needs no more
@@ -805,10 +819,8 @@ int mgc_mlp_train_grad(int64_t n, const float* x, const float* target, const mgc
   if (cudaMemsetAsync(loss, 0, sizeof(float), s) != cudaSuccess) return MGC_E_CUDA;
   const Net net = make_net(w);
   // resident blocks only: each stages the weights once for its tiles
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-    return MGC_E_CUDA;
+  const int sms = sm_count();
+  if (sms < 1) return MGC_E_CUDA;
   const int nb = imin_(grid_for((n + 15) / 16), sms * kTrainBlocks);
   k_mlp_fwd_bwd<<<nb, WARPS * 32, 0, s>>>(n, x, target, net, xb, h1b, dz1b, dz2b, grad, loss,
                                          1.0f / (float)n);
